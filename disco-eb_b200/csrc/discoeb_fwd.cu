@@ -12,6 +12,8 @@
 #include <cstring>
 
 #include "discoeb.h"
+#include "emit_output.cuh"
+#include "solve_block_launch.cuh"
 #include "stepper.cuh"
 
 using namespace dscb;
@@ -28,35 +30,6 @@ __device__ __forceinline__ void copy_cosmo(const WarpTeam& tm, const DiscoebCosm
     tm.sync();
 }
 
-// write state / projected state / output fields of one output time (team-parallel)
-__device__ void emit_output(const WarpTeam& tm, const DiscoebCosmo& P, const Dims& D, double k, double tau,
-                            const double* y, double* yfull, double* y20, double* scratch20)
-{
-    const int n = D.n;
-    double fld[4];
-    const bool rsa = rsa_projection<double>(P, nullptr, D, tau, k, y, nullptr, fld);  // all lanes, identical
-    // projected state into scratch (shared) then outputs
-    double* yp = scratch20;  // n doubles of shared scratch
-    for (int i = tm.lane; i < n; i += 32) {
-        double v = y[i];
-        if (rsa) {
-            const int s = rsa_slot(D, i);
-            if (s >= 0) v = fld[s];
-            else if (s == -1) v = 0.0;
-        }
-        yp[i] = v;
-        if (yfull) yfull[i] = v;
-    }
-    tm.sync();
-    if (y20 && tm.leader()) {
-        double o[20];
-        output_vars<double>(P, nullptr, D, k, yp, nullptr, o);
-        for (int q = 0; q < 20; ++q) y20[q] = o[q];
-    }
-    tm.sync();
-}
-
-// TM: WarpTeam (FP64) or WarpTeamMixed (FP32 chain factors, mix_doubles more per warp)
 template <class TM>
 __global__ void __launch_bounds__(256) fwd_structured_kernel(
     const DiscoebCosmo* __restrict__ cosmos, int n_cosmo, const int32_t* __restrict__ mode_cosmo, DiscoebControl ctrl,
@@ -559,13 +532,20 @@ int32_t discoeb_fwd(const DiscoebCosmo* cosmos_dev, const DiscoebCosmo* cosmo0_h
     if (!(ctrl->rtol > 0.0) || !(ctrl->atol >= 0.0) || ctrl->max_steps < 1) return DISCOEB_EINVAL;
     const Dims D = make_dims(*cosmo0_host);
     const int mem = mode_mem_doubles(D), mix = mixed ? mixed_mem_doubles(D) : 0;
-    const size_t per_warp = (size_t)(kCosmoDoubles + mem + mix) * sizeof(double);
-    const auto kernel = mixed ? fwd_structured_kernel<WarpTeamMixed> : fwd_structured_kernel<WarpTeam>;
+    cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return DISCOEB_ECUDA;
-    int max_optin = 0, n_sm = 0;
+    int max_optin = 0;
     cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    // FP64: a block of warps per mode, up to the number of modes where one warp per mode has more of
+    // them in flight; the same results bit for bit
+    if (!mixed && blk::smem_bytes(D) <= (size_t)max_optin && blk::block_wins(D, n_modes, sms))
+        return blk::launch_fwd(cosmos_dev, n_cosmo, mode_cosmo, *ctrl, n_modes, kmodes, tau_start, y0, switch_tau,
+                               n_out, tau_out, D, y_full, y_out20, status, nsteps, sms, s);
+    const size_t per_warp = (size_t)(kCosmoDoubles + mem + mix) * sizeof(double);
+    const auto kernel = mixed ? fwd_structured_kernel<WarpTeamMixed> : fwd_structured_kernel<WarpTeam>;
     int wpb = ctrl->warps_per_block > 0 ? ctrl->warps_per_block : 1;  // one mode per block: the most resident warps
     if (wpb > 8) wpb = 8;
     while (wpb > 1 && per_warp * wpb > (size_t)max_optin) --wpb;
@@ -574,10 +554,8 @@ int32_t discoeb_fwd(const DiscoebCosmo* cosmos_dev, const DiscoebCosmo* cosmo0_h
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return DISCOEB_ECUDA;
     int blocks = (n_modes + wpb - 1) / wpb;
-    cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     kernel<<<blocks, 32 * wpb, smem, s>>>(cosmos_dev, n_cosmo, mode_cosmo, *ctrl, n_modes, kmodes, tau_start, y0,
                                           switch_tau, n_out, tau_out, mem, mix, y_full, y_out20, status, nsteps);
-    (void)n_sm;
     return cudaGetLastError() == cudaSuccess ? DISCOEB_SUCCESS : DISCOEB_ECUDA;
 }
 

@@ -55,9 +55,20 @@ template <class B> DHD double val(const DualT<B>& x) { return val(x.v); }
 DHD double der(double) { return 0.0; }
 DHD double der(const Dual& x) { return x.d; }
 
+// Reciprocal, square root, exponential and logarithm: inline, or with DSCB_CALL_MATH as calls (the
+// same functions; a translation unit whose kernels are bound by instruction fetch defines it).
+#if defined(__CUDACC__) && defined(DSCB_CALL_MATH)
+static __device__ __noinline__ double call_rcp(double x) { return __drcp_rn(x); }
+static __device__ __noinline__ double call_sqrt(double x) { return sqrt(x); }
+static __device__ __noinline__ double call_exp(double x) { return exp(x); }
+static __device__ __noinline__ double call_log(double x) { return log(x); }
+#endif
+
 DHD double rcp(double x)
 {
-#if defined(__CUDA_ARCH__)
+#if defined(__CUDA_ARCH__) && defined(DSCB_CALL_MATH)
+    return call_rcp(x);
+#elif defined(__CUDA_ARCH__)
     return __drcp_rn(x);
 #else
     return 1.0 / x;
@@ -69,9 +80,15 @@ template <class B> DHD DualT<B> rcp(const DualT<B>& x)
     return DualT<B>(r, -(r * r) * x.d);
 }
 
+#if defined(__CUDA_ARCH__) && defined(DSCB_CALL_MATH)
+DHD double xexp(double x) { return call_exp(x); }
+DHD double xlog(double x) { return call_log(x); }
+DHD double xsqrt(double x) { return call_sqrt(x); }
+#else
 DHD double xexp(double x) { return exp(x); }
 DHD double xlog(double x) { return log(x); }
 DHD double xsqrt(double x) { return sqrt(x); }
+#endif
 DHD double xpow(double x, double p) { return pow(x, p); }
 
 template <class B> DHD DualT<B> xexp(const DualT<B>& x)

@@ -297,11 +297,22 @@ DHD BgTables<T> bg_tables(const TM& tm, const DiscoebCosmo& P, const Par<T>& par
     return r;
 }
 
+// The Friedmann sum 3 (a'/a)^2, in source order; a caller that must reproduce one particular
+// rounding of it (solve_block.cuh) passes its own form to bg_finish.
+struct Friedmann {
+    template <class T>
+    DHD T operator()(const DiscoebCosmo& P, const Par<T>& par, const Bg<T>& b, const BgTables<T>& tb) const
+    {
+        return par.grhom * par.Omegam * b.ia + (P.grhog + P.grhor * (P.Neff + P.Nmnu * tb.rhonu)) * b.ia2 +
+               par.grhom * par.OmegaDE * b.rho_Q * b.a2 + par.grhom * P.Omegak;
+    }
+};
+
 // regime < 0: switches from (tau, a) exactly as model_synchronous evaluates them;
 // otherwise bitmask 1 = RSA, 2 = UFA, 4 = TCA.
-template <class T>
+template <class T, class FR = Friedmann>
 DHD void bg_finish(const DiscoebCosmo& P, const Par<T>& par, T a, const BgTables<T>& tb, double tau, double k,
-                   int regime, Bg<T>& b)
+                   int regime, Bg<T>& b, const FR& friedmann = FR())
 {
     b.par = par;
     b.a = a;
@@ -317,8 +328,7 @@ DHD void bg_finish(const DiscoebCosmo& P, const Par<T>& par, T a, const BgTables
     b.opw = 1.0 + b.w_Q;
     b.iopw = rcp(b.opw);
     b.rho_Q = tb.rho_Q;
-    T grho = par.grhom * par.Omegam * b.ia + (P.grhog + P.grhor * (P.Neff + P.Nmnu * tb.rhonu)) * b.ia2 +
-             par.grhom * par.OmegaDE * b.rho_Q * b.a2 + par.grhom * P.Omegak;
+    T grho = friedmann(P, par, b, tb);
     b.aH = xsqrt(grho * (1.0 / 3.0));
     const T iaH = rcp(b.aH);
     T xeprime = tb.xep * b.aH;

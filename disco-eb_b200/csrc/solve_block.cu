@@ -1,0 +1,172 @@
+// Forward perturbation solve, FP64, a block of warps per mode: kernels and launch of discoeb_fwd.
+#define DSCB_CALL_MATH
+#include <cuda_runtime.h>
+
+#include "discoeb.h"
+#include "emit_output.cuh"
+#include "solve_block.cuh"
+#include "solve_block_launch.cuh"
+
+using namespace dscb;
+
+namespace {
+
+// discoeb_fwd, FP64 form: a block of cooperating warps per mode (solve_block.cuh).  With whole states
+// asked for, the solve stores them as they are and project_states_kernel applies the RSA
+// projection afterwards, one warp per (mode, output): 320 projections per mode would otherwise sit
+// on the mode's chain of steps.
+template <int MaxThreads, int MinBlocks>
+__global__ void __launch_bounds__(MaxThreads, MinBlocks) fwd_block_kernel(
+    const DiscoebCosmo* __restrict__ cosmos, int n_cosmo, const int32_t* __restrict__ mode_cosmo, DiscoebControl ctrl,
+    const double* __restrict__ kmodes, const double* __restrict__ tau_start, const double* __restrict__ y0,
+    const double* __restrict__ sw, int n_out, const double* __restrict__ tau_out, int n0, double* y_full,
+    double* y_out20, int32_t* status, int32_t* nsteps)
+{
+    extern __shared__ double smem[];
+    DiscoebCosmo* P = reinterpret_cast<DiscoebCosmo*>(smem);
+    blk::Shared& S = *reinterpret_cast<blk::Shared*>(smem + blk::kCosmo);
+    double* wmem = smem + blk::kCosmo + blk::kSharedDoubles;
+    const WarpTeam tm{(int)(threadIdx.x & 31)};
+    const int mode = blockIdx.x, warp = threadIdx.x >> 5;
+    const double qnan = __longlong_as_double(0x7ff8000000000000LL);
+    // outputs never reached are filled with NaN so that they cannot pass for data
+    auto fill_nan = [&](int from) {
+        for (int j = from; j < n_out; ++j) {
+            const size_t o = (size_t)mode * n_out + j;
+            if (y_full) for (int i = tm.lane; i < n0; i += 32) y_full[o * n0 + i] = qnan;
+            if (y_out20) for (int i = tm.lane; i < 20; i += 32) y_out20[o * 20 + i] = qnan;
+        }
+    };
+    const int ci = mode_cosmo ? mode_cosmo[mode] : 0;
+    bool bad = ci < 0 || ci >= n_cosmo;  // invalid cosmology index: report, solve nothing
+    if (!bad) {
+        const int* src = reinterpret_cast<const int*>(cosmos + ci);
+        int* dst = reinterpret_cast<int*>(P);
+        for (int i = threadIdx.x; i < (int)(sizeof(DiscoebCosmo) / 4); i += blockDim.x) dst[i] = src[i];
+    }
+    __syncthreads();
+    Dims D{};
+    if (!bad) {
+        D = make_dims(*P);
+        bad = D.n != n0;  // every cosmology must have the sizes of the first
+    }
+    if (bad) {
+        if (warp == 0) fill_nan(0);
+        if (threadIdx.x == 0) {
+            status[mode] = DISCOEB_BAD_INDEX;
+            nsteps[mode] = 0;
+        }
+        return;
+    }
+    const int n = D.n;
+    const ModeMem M = blk::block_carve(wmem, D);
+    const double k = kmodes[mode];
+    for (int i = threadIdx.x; i < n; i += blockDim.x) M.y[i] = y0[(size_t)mode * n + i];
+    const double swm[3] = {sw[3 * mode], sw[3 * mode + 1], sw[3 * mode + 2]};
+    const double* tout = tau_out + (size_t)ci * n_out;  // this cosmology's output times
+    __syncthreads();
+    auto emit = [&](int j, const double* y) {
+        if (!y_full)
+            emit_output(tm, *P, D, k, tout[j], y, nullptr, y_out20 + ((size_t)mode * n_out + j) * 20, M.f);
+    };
+    auto rows = [&](int j, int i, double v) {
+        if (y_full) y_full[((size_t)mode * n_out + j) * n + i] = v;
+    };
+    auto accept = [](double, double, double, int) { return true; };
+    const SolveResult R = blk::solve_mode_block(*P, D, ctrl, k, tau_start[mode], swm, n_out, tout, M, S, emit, rows,
+                                                accept);
+    if (warp == 0) {
+        fill_nan(R.outputs);
+        if (tm.leader()) {
+            status[mode] = R.status;
+            nsteps[mode] = R.steps;
+        }
+    }
+}
+
+// The RSA projection of the states fwd_block_kernel stored (in place), and their output fields when
+// asked for: one warp per (mode, output); rows never reached hold NaN and stay as they are.
+__global__ void __launch_bounds__(128) project_states_kernel(
+    const DiscoebCosmo* __restrict__ cosmos, int n_cosmo, const int32_t* __restrict__ mode_cosmo, long long n_points,
+    const double* __restrict__ kmodes, int n_out, const double* __restrict__ tau_out, int n0, double* y_full,
+    double* y_out20)
+{
+    const long long p = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (p >= n_points) return;
+    const WarpTeam tm{(int)(threadIdx.x & 31)};
+    const int mode = (int)(p / n_out), j = (int)(p - (long long)mode * n_out);
+    const int ci = mode_cosmo ? mode_cosmo[mode] : 0;
+    if (ci < 0 || ci >= n_cosmo) return;
+    const DiscoebCosmo& P = cosmos[ci];
+    const Dims D = make_dims(P);
+    if (D.n != n0) return;
+    double* y = y_full + (size_t)p * n0;
+    if (!(y[0] == y[0])) return;
+    const double k = kmodes[mode], tau = tau_out[(size_t)ci * n_out + j];
+    double fld[4];
+    const bool rsa = rsa_projection<double>(P, nullptr, D, tau, k, y, nullptr, fld);  // all lanes, identical
+    tm.sync();
+    if (rsa)
+        for (int i = tm.lane; i < n0; i += 32) {
+            const int s = rsa_slot(D, i);
+            if (s >= 0) y[i] = fld[s];
+            else if (s == -1) y[i] = 0.0;
+        }
+    tm.sync();
+    if (y_out20 && tm.leader()) {
+        double o[20];
+        output_vars<double>(P, nullptr, D, k, y, nullptr, o);
+        for (int q = 0; q < 20; ++q) y_out20[(size_t)p * 20 + q] = o[q];
+    }
+}
+
+}  // namespace
+
+namespace dscb {
+namespace blk {
+
+size_t smem_bytes(const Dims& D)
+{
+    return block_threads(D) > 512 ? ~(size_t)0 : (size_t)smem_doubles(D) * sizeof(double);
+}
+
+// A mode's solve is a serial chain, so few modes want the shortest chain (this form) and many the
+// most modes in flight (the one-warp form, 8 to 16 per SM against 2 here).  With two blocks per SM
+// the lines cross at 9 modes per SM for 31 rows, 12 for 72, 13.5 for 70 and 26 for 141; the rule
+// stays below all of them.  Milliseconds, block / one-warp: 72 rows 1024 modes 34 / 59, 2048 modes
+// 70 / 62, 6144 modes 215 / 135; 141 rows 2048 modes 73 / 109, 4096 modes 147 / 143, 12288 modes
+// 441 / 410.  Above 256 threads (50-multipole hierarchies) the block form wins at every count: 1200
+// modes 94 / 134, 2400 modes 187 / 259.
+bool block_wins(const Dims& D, int n_modes, int sms)
+{
+    return block_threads(D) > 256 || 8LL * n_modes <= (24LL + D.n) * sms;
+}
+
+int32_t launch_fwd(const DiscoebCosmo* cosmos, int n_cosmo, const int32_t* mode_cosmo, const DiscoebControl& ctrl,
+                   int n_modes, const double* kmodes, const double* tau_start, const double* y0, const double* sw,
+                   int n_out, const double* tau_out, const Dims& D, double* y_full, double* y_out20, int32_t* status,
+                   int32_t* nsteps, int sms, cudaStream_t stream)
+{
+    const size_t smem = smem_bytes(D);
+    const int threads = block_threads(D);
+    // One block per SM has all the registers it asks for, two share the SM but spill.  Milliseconds,
+    // one / two per SM: 300 modes 15.5 / 19.8 (72 rows) and 23.5 / 29.4 (141 rows); 512 modes up to
+    // k = 10, 30.6 / 39.0; 600 modes 26.3 / 22.4 and 30.3 / 31.2; 1024 modes 43 / 34 and 52 / 38.
+    const auto kernel = threads > 256               ? fwd_block_kernel<512, 1>
+                        : 2LL * n_modes <= 7LL * sms ? fwd_block_kernel<256, 1>
+                                                     : fwd_block_kernel<256, 2>;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+        return DISCOEB_ECUDA;
+    kernel<<<n_modes, threads, smem, stream>>>(cosmos, n_cosmo, mode_cosmo, ctrl, kmodes, tau_start, y0, sw, n_out,
+                                        tau_out, D.n, y_full, y_out20, status, nsteps);
+    if (y_full) {
+        const long long points = (long long)n_modes * n_out;
+        project_states_kernel<<<(unsigned)((points + 3) / 4), 128, 0, stream>>>(cosmos, n_cosmo, mode_cosmo, points,
+                                                                                kmodes, n_out, tau_out, D.n, y_full,
+                                                                                y_out20);
+    }
+    return cudaGetLastError() == cudaSuccess ? DISCOEB_SUCCESS : DISCOEB_ECUDA;
+}
+
+}  // namespace blk
+}  // namespace dscb
