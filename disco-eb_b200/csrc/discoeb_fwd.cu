@@ -13,8 +13,10 @@
 
 #include "discoeb.h"
 #include "emit_output.cuh"
+#include "handover.cuh"
 #include "solve_block_launch.cuh"
 #include "stepper.cuh"
+#include "tangent_block_launch.cuh"
 
 using namespace dscb;
 
@@ -108,82 +110,6 @@ __global__ void __launch_bounds__(256) fwd_structured_kernel(
 
 constexpr int kTanDoubles = (sizeof(DiscoebTangent) + 7) / 8;
 constexpr int kMaxDirsPerBlock = 6;
-
-// Output fields and their tangents at output time j of one (mode, direction): the tangent of
-// the state at the moving output time is y' + f tau_out', then the RSA projection and the
-// output conversion in dual numbers.  y: the forward state at tau_out[j]; pf: n doubles of
-// scratch; TT.fd / TT.jk are used as scratch.  Full: the RSA-projected state and its tangent
-// (n values per output) are written instead of the 20 output fields.  Kept out of line: it runs
-// at output times only, and inlined into the tangent loop it lengthens the hot code the seven
-// warps of a block fetch (measured: the gradient kernel 2% slower inlined).
-template <bool Full>
-__device__ __noinline__ void emit_tangent_output(const WarpTeam& tm, const DiscoebCosmo& P, const DiscoebTangent* TN, const Dims& D,
-                                    double k, int mode, int dir, int n_modes, int n_out, int j, const double* tau_out,
-                                    const double* tau_out_dot, const double* y, int regime, const TanMem& TT,
-                                    double* pf, double* y_out20, double* y_out20_dot)
-{
-    const int n = D.n;
-    // f at the output time (left limit of the last step's regime), for the moving output time
-    int hint = P.xe_loga.n_knots / 2;
-    Bg<double> b;
-    bg_eval_team(tm, P, y[0], tau_out[j], k, regime, b, hint);
-    rhs_team(tm, P, D, b, k, tau_out[j], y, TT.fd, (double*)nullptr);
-    tm.sync();
-    const double td = tau_out_dot[(size_t)dir * n_out + j];
-    for (int i = tm.lane; i < n; i += 32) TT.jk[i] = TT.yd[i] + TT.fd[i] * td;
-    tm.sync();
-    Dual fld[4];
-    const bool rsa = rsa_projection<Dual>(P, TN, D, tau_out[j], k, y, TT.jk, fld);
-    for (int i = tm.lane; i < n; i += 32) {
-        double v = y[i], vd = TT.jk[i];
-        if (rsa) {
-            const int sl = rsa_slot(D, i);
-            if (sl >= 0) { v = fld[sl].v; vd = fld[sl].d; }
-            else if (sl == -1) { v = 0.0; vd = 0.0; }
-        }
-        if constexpr (Full) {
-            const size_t oo = (size_t)mode * n_out + j;
-            y_out20_dot[((size_t)dir * n_modes * n_out + oo) * n + i] = vd;
-            if (dir == 0 && y_out20) y_out20[oo * n + i] = v;
-        } else {
-            pf[i] = v;
-            TT.fd[i] = vd;
-        }
-    }
-    tm.sync();
-    if constexpr (Full) return;
-    if (tm.leader()) {
-        Dual o[20];
-        output_vars<Dual>(P, TN, D, k, pf, TT.fd, o);
-        const size_t oo = (size_t)mode * n_out + j;
-        for (int q = 0; q < 20; ++q) y_out20_dot[((size_t)dir * n_modes * n_out + oo) * 20 + q] = o[q].d;
-        if (dir == 0 && y_out20)
-            for (int q = 0; q < 20; ++q) y_out20[oo * 20 + q] = o[q].v;
-    }
-    tm.sync();
-}
-
-// Bounded wait of one warp on a shared-memory counter: lane 0 polls until *flag >= target (or
-// the block's abort flag is set, or the poll budget runs out, after which it sets the abort
-// flag itself); returns true when the target was reached.  No wait can last forever.
-constexpr long long kMaxPolls = 1LL << 24;  // ~2 s with the back-off below; a step takes < 1 ms
-__device__ long long poll_budget(const DiscoebControl& c) { return c.max_polls > 0 ? (long long)c.max_polls : kMaxPolls; }
-__device__ bool wait_at_least(const WarpTeam& tm, volatile int* flag, int target, volatile int* abort_flag,
-                              long long max_polls)
-{
-    int ok = 0;
-    if (tm.leader()) {
-        long long polls = 0;
-        while (true) {
-            if (*flag >= target) { ok = 1; break; }
-            if (*abort_flag) break;
-            if (++polls > max_polls) { *abort_flag = 1; break; }
-            __nanosleep(100);
-        }
-        __threadfence_block();
-    }
-    return __shfl_sync(0xffffffffu, ok, 0) != 0;
-}
 
 // discoeb_jvp: one block per (mode, group of directions).  Warp 0 runs the adaptive forward
 // solve and publishes every accepted step (start state, the 8 stages and the factorisation of
@@ -482,6 +408,17 @@ int32_t launch_jvp(const DiscoebCosmo* cosmos_dev, const DiscoebCosmo* cosmo0_ho
         return DISCOEB_EINVAL;
     if (ctrl->method != DISCOEB_METHOD_RODAS5_STRUCTURED) return DISCOEB_EUNSUPPORTED;
     if (!(ctrl->rtol > 0.0) || !(ctrl->atol >= 0.0) || ctrl->max_steps < 1) return DISCOEB_EINVAL;
+    int dev = 0, max_optin = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return DISCOEB_ECUDA;
+    cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    size_t bsmem = 0;
+    const int bnd = blk::jvp_directions(make_dims(*cosmo0_host), n_dir < kMaxDirsPerBlock ? n_dir : kMaxDirsPerBlock,
+                                        (size_t)max_optin, bsmem);
+    if (bnd > 0)
+        return blk::launch_jvp_block<Full>(cosmos_dev, n_cosmo, mode_cosmo, tangents_dev, n_dir, bnd, bsmem,
+                                           make_dims(*cosmo0_host), *ctrl, n_modes, kmodes, tau_start, y0, y0_dot,
+                                           switch_tau, n_out, tau_out, tau_out_dot, y_out, y_out_dot, status, nsteps,
+                                           reinterpret_cast<cudaStream_t>(stream));
     const JvpPlan plan = jvp_plan(*cosmo0_host, n_dir, n_modes);
     if (plan.dpb < 0) return DISCOEB_ECUDA;
     // the split record is used when the caller passes room for it (discoeb_jvp_records_bytes

@@ -645,24 +645,25 @@ __device__ __forceinline__ bool factor_tri(const Bands& B, int c, int len, Ctl& 
     return ok;
 }
 
-// Forward and back substitution along long chain c (solve_chain) for z (elements ZS apart), with the
+// Forward and back substitution along long chain c (solve_chain) for z (elements ZS apart; the factors
+// ES apart), with the
 // chains' stride NL known at compile time; each element is loaded four steps before its use.
-template <int ZS, int NL>
+template <int ZS, int NL, int ES>
 __device__ __forceinline__ void solve_tri_n(const Bands& B, int c, double al2, double au2, double* z)
 {
-    constexpr int se = 4 * NL, sz = ZS * NL;
+    constexpr int se = ES * NL, sz = ZS * NL;
     extern __shared__ double smem[];  // (indices into it, so that every access is a shared-memory one)
-    int e = (int)(B.E - smem) + 4 * c, zp = (int)(z - smem) + ZS * c;
+    int e = (int)(B.E - smem) + ES * c, zp = (int)(z - smem) + ZS * c;
     const int extra = B.steps * NL;
-    const double* e5 = B.E + 4 * (extra + 4);
+    const double* e5 = B.E + ES * (extra + 4);
     double* z5 = z + ZS * (extra + 4);
     double* z8 = z + ZS * B.row8;
     double v5 = 0.0, v6 = 0.0, v7 = 0.0;
     if (c == 0) {
         v5 = z5[0];
-        v6 = z5[ZS] - e5[4 + E_LO] * v5;
-        v7 = z5[2 * ZS] - e5[8 + E_LO] * v6;
-        double v8 = *z8 - B.E[4 * B.row8 + E_LO] * v7;
+        v6 = z5[ZS] - e5[ES + E_LO] * v5;
+        v7 = z5[2 * ZS] - e5[2 * ES + E_LO] * v6;
+        double v8 = *z8 - B.E[ES * B.row8 + E_LO] * v7;
         v8 -= al2 * v6;
         *z8 = v8;
     }
@@ -708,10 +709,10 @@ __device__ __forceinline__ void solve_tri_n(const Bands& B, int c, double al2, d
         e -= 4 * se;
     }
     if (c == 0) {
-        const double x8 = *z8, x7 = (v7 - e5[8 + E_UP] * x8) * e5[8 + E_DI];
-        double x6 = v6 - e5[4 + E_UP] * x7;
+        const double x8 = *z8, x7 = (v7 - e5[2 * ES + E_UP] * x8) * e5[2 * ES + E_DI];
+        double x6 = v6 - e5[ES + E_UP] * x7;
         x6 -= au2 * x8;
-        x6 *= e5[4 + E_DI];
+        x6 *= e5[ES + E_DI];
         z5[2 * ZS] = x7;
         z5[ZS] = x6;
         z5[0] = (v5 - e5[E_UP] * x6) * e5[E_DI];
@@ -719,22 +720,22 @@ __device__ __forceinline__ void solve_tri_n(const Bands& B, int c, double al2, d
 }
 // The same with the number of positions known too: the forward results stay in registers, and every
 // load is issued ahead of the dependent arithmetic (20 positions: 1490 -> ~800 cycles).
-template <int ZS, int NL, int STEPS>
+template <int ZS, int NL, int STEPS, int ES>
 __device__ __forceinline__ void solve_tri_s(const Bands& B, int c, double al2, double au2, double* z)
 {
     extern __shared__ double smem[];
-    constexpr int se = 4 * NL, sz = ZS * NL, extra = STEPS * NL;
-    const int e = (int)(B.E - smem) + 4 * c, zp = (int)(z - smem) + ZS * c;
-    const double* e5 = B.E + 4 * (extra + 4);
+    constexpr int se = ES * NL, sz = ZS * NL, extra = STEPS * NL;
+    const int e = (int)(B.E - smem) + ES * c, zp = (int)(z - smem) + ZS * c;
+    const double* e5 = B.E + ES * (extra + 4);
     double* z5 = z + ZS * (extra + 4);
     double* z8 = z + ZS * B.row8;
     double v6 = 0.0, v7 = 0.0;
     const bool photon = c == 0;
     if (photon) {
         const double v5 = z5[0];
-        v6 = z5[ZS] - e5[4 + E_LO] * v5;
-        v7 = z5[2 * ZS] - e5[8 + E_LO] * v6;
-        double v8 = *z8 - B.E[4 * B.row8 + E_LO] * v7;
+        v6 = z5[ZS] - e5[ES + E_LO] * v5;
+        v7 = z5[2 * ZS] - e5[2 * ES + E_LO] * v6;
+        double v8 = *z8 - B.E[ES * B.row8 + E_LO] * v7;
         v8 -= al2 * v6;
         *z8 = v8;
     }
@@ -754,21 +755,21 @@ __device__ __forceinline__ void solve_tri_s(const Bands& B, int c, double al2, d
 #pragma unroll
     for (int p = 0; p < STEPS; ++p) smem[zp + p * sz] = v[p];
     if (photon) {
-        const double v5 = z5[0], x8 = *z8, x7 = (v7 - e5[8 + E_UP] * x8) * e5[8 + E_DI];
-        double x6 = v6 - e5[4 + E_UP] * x7;
+        const double v5 = z5[0], x8 = *z8, x7 = (v7 - e5[2 * ES + E_UP] * x8) * e5[2 * ES + E_DI];
+        double x6 = v6 - e5[ES + E_UP] * x7;
         x6 -= au2 * x8;
-        x6 *= e5[4 + E_DI];
+        x6 *= e5[ES + E_DI];
         z5[2 * ZS] = x7;
         z5[ZS] = x6;
         z5[0] = (v5 - e5[E_UP] * x6) * e5[E_DI];
     }
 }
-template <int ZS> __device__ __forceinline__ void solve_tri(const Bands& B, int c, double al2, double au2, double* z)
+template <int ZS, int ES = 4> __device__ __forceinline__ void solve_tri(const Bands& B, int c, double al2, double au2, double* z)
 {
-    if (B.nl != kNarrow) solve_tri_n<ZS, kWide>(B, c, al2, au2, z);
-    else if (B.steps == 20) solve_tri_s<ZS, kNarrow, 20>(B, c, al2, au2, z);
-    else if (B.steps == 12) solve_tri_s<ZS, kNarrow, 12>(B, c, al2, au2, z);
-    else solve_tri_n<ZS, kNarrow>(B, c, al2, au2, z);
+    if (B.nl != kNarrow) solve_tri_n<ZS, kWide, ES>(B, c, al2, au2, z);
+    else if (B.steps == 20) solve_tri_s<ZS, kNarrow, 20, ES>(B, c, al2, au2, z);
+    else if (B.steps == 12) solve_tri_s<ZS, kNarrow, 12, ES>(B, c, al2, au2, z);
+    else solve_tri_n<ZS, kNarrow, ES>(B, c, al2, au2, z);
 }
 
 // ---- the special rows and metric functionals (special_part, the momentum bins in a loop) ----
@@ -818,16 +819,15 @@ __device__ __forceinline__ void neutrino_sums(const WarpTeam& tm, const DiscoebC
     fnu = Dual(tm.bcast(s, 4), 0.0);
 }
 
+// special_part from the sums over the momentum bins
 template <class T, class S, class PR>
-__device__ __forceinline__ void special_block(const WarpTeam& tm, const DiscoebCosmo& P, const Dims& D, const Bg<T>& b,
-                                              double k, double tau, StateAt Y, const T* bins, T sp[15], T& g0, T& g1,
-                                              T& g2)
+__device__ __forceinline__ void special_core(const DiscoebCosmo& P, const Dims& D, const Bg<T>& b, double k, double tau,
+                                             StateAt Y, const T& drho, T dp, const T& fnu, T sp[15], T& g0, T& g1,
+                                             T& g2)
 {
-    const int n = D.n, nq = D.nq, iq0 = D.iq0, idxr = D.idxr;
+    const int n = D.n, idxr = D.idxr;
     const double k2 = k * k;
     const T Omegac = b.par.Omegam - b.par.Omegab;
-    T drho = 0.0, dp = 0.0, fnu = 0.0;
-    neutrino_sums(tm, P, nq, Y.base + iq0, bins, drho, dp, fnu);
     dp = dp * (1.0 / 3.0);
     const S eta = Y(2), deltac = Y(3), thetac = Y(4), deltab = Y(5), thetab = Y(6);
     const S deltag = Y(7), thetag = Y(8), y9 = Y(9);
@@ -895,6 +895,16 @@ __device__ __forceinline__ void special_block(const WarpTeam& tm, const DiscoebC
     g0 = H;
     g1 = E;
     g2 = polter;
+}
+
+template <class T, class S, class PR>
+__device__ __forceinline__ void special_block(const WarpTeam& tm, const DiscoebCosmo& P, const Dims& D, const Bg<T>& b,
+                                              double k, double tau, StateAt Y, const T* bins, T sp[15], T& g0, T& g1,
+                                              T& g2)
+{
+    T drho = 0.0, dp = 0.0, fnu = 0.0;
+    neutrino_sums(tm, P, D.nq, Y.base + D.iq0, bins, drho, dp, fnu);
+    special_core<T, S, PR>(P, D, b, k, tau, Y, drho, dp, fnu, sp, g0, g1, g2);
 }
 
 // ---- one row per thread: warps "rows" (hierarchy rows) and the lanes of "special" ----
@@ -1083,17 +1093,17 @@ __device__ __forceinline__ void slot_sums(const WarpTeam& tm, const Slots& sl, c
 }
 
 // the two short chains: CDM (rows 3, 4) and dark energy
-__device__ __forceinline__ double* short_chain(const Bands& B, int which)
+template <int ES = 4> __device__ __forceinline__ double* short_chain(const Bands& B, int which)
 {
-    return B.E + 4 * (B.steps * B.nl + (which ? 7 : 2));
+    return B.E + ES * (B.steps * B.nl + (which ? 7 : 2));
 }
-template <int ZS> __device__ __forceinline__ void solve_short(const Bands& B, int lane, double* z, int nrhs)
+template <int ZS, int ES = 4> __device__ __forceinline__ void solve_short(const Bands& B, int lane, double* z, int nrhs)
 {
     if (lane < 2 * nrhs) {
-        const double* c = short_chain(B, lane & 1);
+        const double* c = short_chain<ES>(B, lane & 1);
         double* v = z + (lane >> 1) * B.pc + ZS * (B.steps * B.nl + ((lane & 1) ? 7 : 2));
-        const double b = v[ZS] - c[4 + E_LO] * v[0];
-        const double x1 = b * c[4 + E_DI];
+        const double b = v[ZS] - c[ES + E_LO] * v[0];
+        const double x1 = b * c[ES + E_DI];
         v[ZS] = x1;
         v[0] = (v[0] - c[E_UP] * x1) * c[E_DI];
     }
@@ -1343,19 +1353,28 @@ __device__ __forceinline__ void chain_step(const WarpTeam& tm, const Dims& D, Sh
     }
 }
 
+// publish() of a solve whose steps nobody records
+struct NoPublish {
+    __device__ __forceinline__ void copy(int, int, double, const ModeMem&, const Bands&, int, int) const {}
+    __device__ __forceinline__ void done(const ModeMem&) const {}
+};
+
 // The solve.  y0 is in M.y; emit(j, y, regime) runs on warp 0 with the state exactly at tout[j];
 // rows(j, i, y_i) runs on the thread that owns row i (either may do nothing); accept as in
-// solve_mode, on warp 0.  Every thread of the block calls it; the result is valid on warp 0.
-template <class Emit, class Rows, class Accept>
+// solve_mode, on warp 0.  After an accepted step, publish.copy(row, position, y, M, B, thread,
+// threads) runs on every thread of special + rows while M still holds the step (all but row 0, whose
+// next stages are under way), and publish.done(M) on warp 0 when all of them are through.  Every thread of the block calls it; the result is valid on warp 0.
+template <class Emit, class Rows, class Accept, class Publish = NoPublish>
 __device__ __forceinline__ SolveResult solve_mode_block(const DiscoebCosmo& P, const Dims& D, const DiscoebControl& C,
                                                         double k, double t0, const double* sw, int nout,
                                                         const double* tout, const ModeMem& M, Shared& S, Emit& emit,
-                                                        Rows& rows, Accept& accept)
+                                                        Rows& rows, Accept& accept,
+                                                        const Publish& publish = Publish())
 {
     const int warp = threadIdx.x >> 5;
     const WarpTeam tm{(int)(threadIdx.x & 31)};
     const int n = D.n, nrw = row_warps(D);
-    const int c_rows = 32 * (1 + nrw), c_all = c_rows + 32;
+    const int c_rows = 32 * (1 + nrw), c_all = c_rows + 32, c_solve = c_all + 64;
     const Bands B = make_bands(D, M.A);
     SolveResult R = {DISCOEB_OK, 0, 0, 0};
     int hint = P.xe_loga.n_knots / 2;
@@ -1369,7 +1388,7 @@ __device__ __forceinline__ SolveResult solve_mode_block(const DiscoebCosmo& P, c
         bar_sync(2, 64);
         prep_point(tm, scale, P, D, k, M.y[0], t0, regime_at(P, t0, sw), S.pt[0], hint);
         for (;;) {
-            __syncthreads();
+            bar_sync(0, c_solve);
             if (!S.c.go) break;
             if (S.c.accepted) cur ^= 1;
             helper_step(tm, scale, P, D, k, sw, C, S, cur, M, c_rows + 32, hint, iv);
@@ -1382,7 +1401,7 @@ __device__ __forceinline__ SolveResult solve_mode_block(const DiscoebCosmo& P, c
             B.Z[x] = 0.0;
         }
         for (;;) {
-            __syncthreads();
+            bar_sync(0, c_solve);
             if (!S.c.go) break;
             chain_step(tm, D, S, B, c_all);
         }
@@ -1511,17 +1530,19 @@ __device__ __forceinline__ SolveResult solve_mode_block(const DiscoebCosmo& P, c
                 if (keep) S.c.y0_next = M.u[0] + M.K[7 * n];
             }
         }
-        __syncthreads();
+        bar_sync(0, c_solve);
         first = false;
         const int go = S.c.go, accepted = S.c.accepted;
         if (accepted) {
             cur ^= 1;
+            publish.copy(W.i, W.pos, W.y, M, B, special ? tm.lane : 32 * (warp - 1) + tm.lane, c_rows);
             // the state advances; each thread its own row
             if (W.i >= 0) {
                 W.y = W.i == 0 ? S.c.y0_next : W.u + M.K[7 * n + W.i];
                 M.y[W.i] = W.y;
             }
             bar_sync(1, c_rows);
+            if (special) publish.done(M);
             const double tacc = go ? S.c.t : S.c.tnext;
             while (iout < nout && t_out <= tacc) {
                 if (special) emit(iout, M.y);
