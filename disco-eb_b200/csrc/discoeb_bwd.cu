@@ -1,7 +1,8 @@
 // Discrete adjoint on sm_100a: the recording forward solve, the reverse sweep and the contraction
 // of the cotangents with parameter tangents; C ABI (include/discoeb.h).
 //
-// Layout: the recording forward is the forward solve (one warp per k-mode) whose accept hook
+// Layout: the recording forward is the forward solve (solve_block.cu; above its line of modes, one
+// warp per k-mode) whose accept hook
 // writes each accepted step's end time (8 bytes) and every checkpoint_every-th start state into
 // the caller's record buffer.  The reverse sweep runs one block of five warps per mode (replay of
 // the segments from their checkpoints, recomputation of each step, the chain of the cotangents of
@@ -18,6 +19,7 @@
 
 #include "adjoint.cuh"
 #include "discoeb.h"
+#include "solve_block_launch.cuh"
 
 using namespace dscb;
 
@@ -541,9 +543,19 @@ int32_t discoeb_fwd_record(const DiscoebCosmo* cosmos_dev, const DiscoebCosmo* c
     if (cudaGetDevice(&dev) != cudaSuccess) return DISCOEB_ECUDA;
     cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     if (smem > (size_t)max_optin) return DISCOEB_EUNSUPPORTED;
+    const long long rec = record_doubles(D.n, step_capacity, checkpoint_every);
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    // a block of warps per mode, as in discoeb_fwd (32 modes to k = 1: 44.6 -> 9.9 ms), bit for bit the
+    // same; many modes keep a warp each (block_wins)
+    if (blk::smem_bytes(D) <= (size_t)max_optin && blk::block_wins(D, n_modes, sms)) {
+        const blk::StepRecords r{records, rec, step_capacity, checkpoint_every, n_accepted};
+        return blk::launch_fwd(cosmos_dev, n_cosmo, mode_cosmo, *ctrl, n_modes, kmodes, tau_start, y0, switch_tau,
+                               n_out, tau_out, D, nullptr, y_out20, status, nsteps, &r, sms,
+                               reinterpret_cast<cudaStream_t>(stream));
+    }
     if (cudaFuncSetAttribute(fwd_record_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return DISCOEB_ECUDA;
-    const long long rec = record_doubles(D.n, step_capacity, checkpoint_every);
     const int blocks = (n_modes + wpb - 1) / wpb;
     fwd_record_kernel<<<blocks, 32 * wpb, smem, reinterpret_cast<cudaStream_t>(stream)>>>(
         cosmos_dev, n_cosmo, mode_cosmo, *ctrl, n_modes, kmodes, tau_start, y0, switch_tau, n_out, tau_out, mem,

@@ -411,6 +411,8 @@ int32_t launch_jvp(const DiscoebCosmo* cosmos_dev, const DiscoebCosmo* cosmo0_ho
     int dev = 0, max_optin = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return DISCOEB_ECUDA;
     cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    // the block form wherever one direction fits beside the forward (fewer than six per block above
+    // ~150 rows: 219 rows one, and still 214 -> 63 ms for 80 modes); larger states keep the form below
     size_t bsmem = 0;
     const int bnd = blk::jvp_directions(make_dims(*cosmo0_host), n_dir < kMaxDirsPerBlock ? n_dir : kMaxDirsPerBlock,
                                         (size_t)max_optin, bsmem);
@@ -480,7 +482,7 @@ int32_t discoeb_fwd(const DiscoebCosmo* cosmos_dev, const DiscoebCosmo* cosmo0_h
     // them in flight; the same results bit for bit
     if (!mixed && blk::smem_bytes(D) <= (size_t)max_optin && blk::block_wins(D, n_modes, sms))
         return blk::launch_fwd(cosmos_dev, n_cosmo, mode_cosmo, *ctrl, n_modes, kmodes, tau_start, y0, switch_tau,
-                               n_out, tau_out, D, y_full, y_out20, status, nsteps, sms, s);
+                               n_out, tau_out, D, y_full, y_out20, status, nsteps, nullptr, sms, s);
     const size_t per_warp = (size_t)(kCosmoDoubles + mem + mix) * sizeof(double);
     const auto kernel = mixed ? fwd_structured_kernel<WarpTeamMixed> : fwd_structured_kernel<WarpTeam>;
     int wpb = ctrl->warps_per_block > 0 ? ctrl->warps_per_block : 1;  // one mode per block: the most resident warps

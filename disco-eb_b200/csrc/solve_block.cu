@@ -15,12 +15,16 @@ namespace {
 // asked for, the solve stores them as they are and project_states_kernel applies the RSA
 // projection afterwards, one warp per (mode, output): 320 projections per mode would otherwise sit
 // on the mode's chain of steps.
-template <int MaxThreads, int MinBlocks>
+//
+// Record: the recording forward of the adjoint.  Each accepted step's end time and every `every`-th
+// start state go into the mode's record (record_doubles), by the controller's warp before the state
+// advances.
+template <int MaxThreads, int MinBlocks, bool Record>
 __global__ void __launch_bounds__(MaxThreads, MinBlocks) fwd_block_kernel(
     const DiscoebCosmo* __restrict__ cosmos, int n_cosmo, const int32_t* __restrict__ mode_cosmo, DiscoebControl ctrl,
     const double* __restrict__ kmodes, const double* __restrict__ tau_start, const double* __restrict__ y0,
     const double* __restrict__ sw, int n_out, const double* __restrict__ tau_out, int n0, double* y_full,
-    double* y_out20, int32_t* status, int32_t* nsteps)
+    double* y_out20, int32_t* status, int32_t* nsteps, blk::StepRecords rec)
 {
     extern __shared__ double smem[];
     DiscoebCosmo* P = reinterpret_cast<DiscoebCosmo*>(smem);
@@ -55,6 +59,7 @@ __global__ void __launch_bounds__(MaxThreads, MinBlocks) fwd_block_kernel(
         if (threadIdx.x == 0) {
             status[mode] = DISCOEB_BAD_INDEX;
             nsteps[mode] = 0;
+            if constexpr (Record) rec.n_accepted[mode] = 0;
         }
         return;
     }
@@ -66,20 +71,34 @@ __global__ void __launch_bounds__(MaxThreads, MinBlocks) fwd_block_kernel(
     const double* tout = tau_out + (size_t)ci * n_out;  // this cosmology's output times
     __syncthreads();
     auto emit = [&](int j, const double* y) {
-        if (!y_full)
+        if (!y_full && (!Record || y_out20))
             emit_output(tm, *P, D, k, tout[j], y, nullptr, y_out20 + ((size_t)mode * n_out + j) * 20, M.f);
     };
     auto rows = [&](int j, int i, double v) {
         if (y_full) y_full[((size_t)mode * n_out + j) * n + i] = v;
     };
-    auto accept = [](double, double, double, int) { return true; };
+    int count = 0;
+    auto accept = [&](double, double, double tnext, int) {
+        if constexpr (Record) {
+            if (count >= rec.cap) return false;
+            double* r = rec.base + (size_t)mode * rec.doubles;
+            if (count % rec.every == 0) {
+                double* c = r + rec.cap + (size_t)(count / rec.every) * n;
+                for (int i = tm.lane; i < n; i += 32) c[i] = M.y[i];
+            }
+            if (tm.leader()) r[count] = tnext;
+            ++count;
+        }
+        return true;
+    };
     const SolveResult R = blk::solve_mode_block(*P, D, ctrl, k, tau_start[mode], swm, n_out, tout, M, S, emit, rows,
                                                 accept);
     if (warp == 0) {
         fill_nan(R.outputs);
         if (tm.leader()) {
-            status[mode] = R.status;
+            status[mode] = (Record && R.status == DISCOEB_ABORTED && count >= rec.cap) ? DISCOEB_RECORD_FULL : R.status;
             nsteps[mode] = R.steps;
+            if constexpr (Record) rec.n_accepted[mode] = count;
         }
     }
 }
@@ -145,20 +164,25 @@ bool block_wins(const Dims& D, int n_modes, int sms)
 int32_t launch_fwd(const DiscoebCosmo* cosmos, int n_cosmo, const int32_t* mode_cosmo, const DiscoebControl& ctrl,
                    int n_modes, const double* kmodes, const double* tau_start, const double* y0, const double* sw,
                    int n_out, const double* tau_out, const Dims& D, double* y_full, double* y_out20, int32_t* status,
-                   int32_t* nsteps, int sms, cudaStream_t stream)
+                   int32_t* nsteps, const StepRecords* records, int sms, cudaStream_t stream)
 {
     const size_t smem = smem_bytes(D);
     const int threads = block_threads(D);
     // One block per SM has all the registers it asks for, two share the SM but spill.  Milliseconds,
     // one / two per SM: 300 modes 15.5 / 19.8 (72 rows) and 23.5 / 29.4 (141 rows); 512 modes up to
     // k = 10, 30.6 / 39.0; 600 modes 26.3 / 22.4 and 30.3 / 31.2; 1024 modes 43 / 34 and 52 / 38.
-    const auto kernel = threads > 256               ? fwd_block_kernel<512, 1>
-                        : 2LL * n_modes <= 7LL * sms ? fwd_block_kernel<256, 1>
-                                                     : fwd_block_kernel<256, 2>;
+    const auto pick = [&](auto one, auto two, auto wide) {
+        return threads > 256 ? wide : 2LL * n_modes <= 7LL * sms ? one : two;
+    };
+    const auto kernel = records ? pick(fwd_block_kernel<256, 1, true>, fwd_block_kernel<256, 2, true>,
+                                       fwd_block_kernel<512, 1, true>)
+                                : pick(fwd_block_kernel<256, 1, false>, fwd_block_kernel<256, 2, false>,
+                                       fwd_block_kernel<512, 1, false>);
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return DISCOEB_ECUDA;
     kernel<<<n_modes, threads, smem, stream>>>(cosmos, n_cosmo, mode_cosmo, ctrl, kmodes, tau_start, y0, sw, n_out,
-                                        tau_out, D.n, y_full, y_out20, status, nsteps);
+                                        tau_out, D.n, y_full, y_out20, status, nsteps,
+                                        records ? *records : StepRecords{});
     if (y_full) {
         const long long points = (long long)n_modes * n_out;
         project_states_kernel<<<(unsigned)((points + 3) / 4), 128, 0, stream>>>(cosmos, n_cosmo, mode_cosmo, points,

@@ -1,4 +1,4 @@
-// Launch of the block solver (solve_block.cuh) for discoeb_fwd.
+// Launch of the block solver (solve_block.cuh) for discoeb_fwd and discoeb_fwd_record.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -17,11 +17,21 @@ size_t smem_bytes(const Dims& D);
 // whether the block form solves n_modes modes on a device of that many SMs faster than a warp per mode
 bool block_wins(const Dims& D, int n_modes, int sms);
 
-// discoeb_fwd's FP64 solve (arguments checked by the caller); a DISCOEB_* status
+// where discoeb_fwd_record's steps go: per mode `doubles` from base on, cap end times, then a start
+// state every `every` steps
+struct StepRecords {
+    double* base;
+    long long doubles;
+    int cap, every;
+    int32_t* n_accepted;
+};
+
+// the FP64 solve of discoeb_fwd and, with records, of discoeb_fwd_record (arguments checked by the
+// caller); a DISCOEB_* status
 int32_t launch_fwd(const DiscoebCosmo* cosmos, int n_cosmo, const int32_t* mode_cosmo, const DiscoebControl& ctrl,
                    int n_modes, const double* kmodes, const double* tau_start, const double* y0, const double* sw,
                    int n_out, const double* tau_out, const Dims& D, double* y_full, double* y_out20, int32_t* status,
-                   int32_t* nsteps, int sms, cudaStream_t stream);
+                   int32_t* nsteps, const StepRecords* records, int sms, cudaStream_t stream);
 
 }  // namespace blk
 }  // namespace dscb

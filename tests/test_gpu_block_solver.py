@@ -66,3 +66,23 @@ def test_gpu_wide_block_solve_matches_oracle(torch_cuda, size):
                                        de_guard_eps=1e-9, return_full=False, **dict(zip(NAMES, size)))
     for idx in (0, 2, 4, 6, 8, 10):  # the same step sequence: agreement far below the solver's tolerance
         np.testing.assert_allclose(y[:, :, idx], yo[:, :, idx], rtol=1e-6, atol=1e-12)
+
+
+# the recording solve of the adjoint: 12 modes on a block each, the same modes in a batch of a warp each
+@pytest.mark.parametrize("every", [1, 7])
+@pytest.mark.parametrize("size", [(3, 3, 3, 3, 1), (11, 11, 11, 8, 3)])
+def test_gpu_recorded_block_and_one_warp_solves_are_the_same(torch_cuda, size, every):
+    import math
+    from discoeb_b200.gradients import AdjointProblem
+    theta = dict(omega_c=0.120, omega_b=0.0224, h=0.674, n_s=0.965, ln10As=math.log(21.0), w0=-0.9, wa=0.1, m_nu=0.06)
+    ks = np.geomspace(1e-3, 0.5, 12)
+    out = []
+    for k in (ks, np.tile(ks, 160)):  # 1920 modes: above both sizes' line
+        p = AdjointProblem(theta, aexp_out=np.array([0.5, 1.0]), kmodes=k, rtol=1e-4, atol=1e-6, checkpoint_every=every,
+                           **dict(zip(NAMES, size)))
+        p.launch_forward()
+        P, status, _ = p.forward_power()
+        assert (status == 0).all()
+        out.append((P[0][:12], np.sort(p.d_nacc.cpu().numpy())[::len(k) // 12]))
+    np.testing.assert_array_equal(out[0][0], out[1][0])
+    np.testing.assert_array_equal(out[0][1], out[1][1])
