@@ -14,6 +14,8 @@
 //      sums with tcgen05.ld and store them (write-only, so a level boundary costs the tensor
 //      cores one TMEM drain, not a read-modify-write of FP64 partials in DRAM)
 //   4. reduce_kernel: C = the scaled sum over levels and K ranges
+// Large products with 6 or 7 slices take residues instead of digits in steps 2 to 4 (residue_kernel,
+// gemm_kernel<true>, crt_kernel), in chunks that reuse the planes' storage.
 // Every wait on a barrier is bounded in time; a CTA whose wait runs out sets the error flag,
 // lets its issued copies and MMAs finish, frees its TMEM and returns, and the reduction then
 // writes NaN into C.
@@ -313,12 +315,223 @@ __global__ void slice_kernel(int rows, int k, const double* __restrict__ X, long
     }
 }
 
+// ---- the product in residues ------------------------------------------------------------------
+
+// 6 and 7 slices multiply 21 and 28 pairs of digit planes.  The same integers (x in units of the last
+// digit, |v| < 2^(7 slices)) have an exact product C with |C| <= k v^2, which its residues modulo 13 or
+// 15 coprime numbers <= 256 determine (the Chinese remainder theorem; for matrix products on integer
+// units: Ozaki, Uchino & Imamura, arXiv:2504.08009): one plane product per modulus instead of one per
+// digit pair, and no dropped levels.  The planes take the digits' place in the workspace, `slices` at
+// most at a time.
+constexpr int kModuli[16] = {256, 253, 251, 247, 241, 239, 233, 229, 227, 223, 217, 211, 199, 197, 193, 191};
+
+struct Crt {
+    int n;                                  // moduli
+    int m[16], w[16];                       // and the inverse of (M / m) modulo m, folded into B's residues
+    float inv[16];
+    double M[3], P[16][3];                  // their product M and M / m, in limbs of 39 bits
+};
+
+// The residue form of this product, or n = 0 where the digit pairs are the better.  A residue plane
+// costs a pass over the operand's doubles per chunk and a drain of the accumulators per plane, so the
+// products must be a third fewer (6 and 7 slices) and many: milliseconds, digits / residues, at
+// 41280 (256 x 256 x 128) units 8.7 / 6.1, at 10400 2.6 / 2.2, at 2600 1.08 / 0.94, at 256 0.25 / 0.31.
+// v is an exact integer below 2^51 (7 slices at most), a K range at most 16512 long (gemm_kernel's
+// quotients).  The error against 64 bits is a quarter of the digits' (no dropped levels).
+Crt residue_form(const Geo& g)
+{
+    Crt c{};
+    const int slices = g.slices, range = (g.kst + g.split - 1) / g.split * BKB;
+    if (slices > 7 || g.split > 4 || (long long)g.mt * g.nt * g.kst < 2500) return c;
+    const double bits = 14.0 * slices + std::log2((double)g.k) + 1.25;
+    double have = 0.0;
+    int n = 0;
+    while (n < 16 && have < bits) have += std::log2((double)kModuli[n++]);
+    if (have < bits || range > 16512 || 3 * n > slices * (slices + 1)) return c;
+    c.n = n;
+    auto limbs = [](unsigned __int128 x, double (&o)[3]) {
+        for (int i = 0; i < 3; ++i) o[i] = (double)(uint64_t)((x >> (39 * i)) & (((unsigned __int128)1 << 39) - 1));
+        o[2] += (double)(uint64_t)(x >> 117) * 0x1p39;
+    };
+    unsigned __int128 M = 1;
+    for (int i = 0; i < n; ++i) M *= (unsigned)kModuli[i];
+    limbs(M, c.M);
+    for (int i = 0; i < n; ++i) {
+        const int m = kModuli[i];
+        c.m[i] = m;
+        c.inv[i] = 1.0f / (float)m;
+        limbs(M / (unsigned)m, c.P[i]);
+        const int r = (int)(M / (unsigned)m % (unsigned)m);
+        int w = 1;
+        while (w * r % m != 1) ++w;
+        c.w[i] = w;
+    }
+    return c;
+}
+
+struct Chunk {
+    int n;
+    float m[kMaxSlices], inv[kMaxSlices];
+    float c17[kMaxSlices], c34[kMaxSlices];  // 2^17 and 2^34 modulo m, nearest to zero
+    float w[kMaxSlices];                     // 0 for A's planes
+};
+void set_modulus(Chunk& c, int i, int m)
+{
+    auto near0 = [&](long long x) { const int r = (int)(x % m); return (float)(2 * r > m ? r - m : r); };
+    c.m[i] = (float)m;
+    c.inv[i] = 1.0f / (float)m;
+    c.c17[i] = near0(1ll << 17);
+    c.c34[i] = near0(1ll << 34);
+}
+
+constexpr float kRoundF = 12582912.0f;  // 1.5 2^23: adding it rounds to an integer, its low byte the integer's
+// t modulo m for an integer |t| < 2^24, nearest to zero up to the quotient's rounding: |r| <= (m + 1) / 2,
+// a signed byte for m <= 253; for m = 256 the quotient is exact and the two ends are the same byte
+__device__ __forceinline__ float residue(float t, float m, float inv)
+{
+    return __fmaf_rn(-m, __fadd_rn(__fmaf_rn(t, inv, kRoundF), -kRoundF), t);
+}
+
+// slice_kernel's layout with the residues of the chunk's moduli for planes, in its thread order (a
+// transposed operand: rows first, so that a load reads 32 consecutive doubles).  What bounds it are the
+// loads, 32 cache lines an instruction: pairs of doubles where the operand's alignment allows them
+// halve those (8192 x 16386, five moduli: 0.61 -> 0.48 ms; staging the rows through shared memory
+// took 1.29).  v, below 2^49, is cut into three signed parts of 17 bits, whose residues sum below 2^24:
+// single precision, exactly.
+__global__ void __launch_bounds__(256)
+    residue_kernel(int rows, int k, const double* __restrict__ X, long long ld, bool trans, bool pairs,
+                   const int* __restrict__ e, const double* __restrict__ scale, int kst, long long n_units, int bits,
+                   Chunk c, size_t plane, uint8_t* __restrict__ D)
+{
+    const long long u = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (u >= n_units) return;
+    const int lo = (int)(u & 2047), rr = lo & 7;
+    const int ch = trans ? lo >> 8 : (lo >> 3) & 7, g = trans ? (lo >> 3) & 31 : lo >> 6;
+    const unsigned rest = (unsigned)(u >> 11);
+    const int kc = (int)(rest % (unsigned)kst);
+    const long long rb = rest / (unsigned)kst;
+    const long long row = rb * 256 + g * 8 + rr;
+    const long long k0 = (long long)kc * BKB + ch * 16;
+    const bool live = row < rows && isfinite(scale[row]) && scale[row] != 0.0;
+    const int sh = bits - (live ? e[row] : 0), sh1 = sh / 2;
+    const double f1 = ldexp(1.0, sh1), f2 = ldexp(1.0, sh - sh1);
+    constexpr double kRound = 6755399441055744.0;  // 1.5 2^52
+    double in[16];
+    if (live && pairs && k0 + 16 <= k) {
+        const double2* p = reinterpret_cast<const double2*>(X + (size_t)row * ld + k0);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const double2 d = p[j];
+            in[2 * j] = d.x;
+            in[2 * j + 1] = d.y;
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+            in[j] = (live && k0 + j < k) ? (trans ? X[(size_t)(k0 + j) * ld + row] : X[(size_t)row * ld + k0 + j]) : 0.0;
+    }
+    float p0[16], p1[16], p2[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+        const double x = in[j];
+        const double v = __dsub_rn(__dadd_rn(x * f1 * f2, kRound), kRound);
+        const double a = __dsub_rn(__dadd_rn(v * 0x1p-34, kRound), kRound), v1 = __fma_rn(-0x1p34, a, v);
+        const double b = __dsub_rn(__dadd_rn(v1 * 0x1p-17, kRound), kRound);
+        p2[j] = (float)a;
+        p1[j] = (float)b;
+        p0[j] = (float)__fma_rn(-0x1p17, b, v1);
+    }
+    uint8_t* dst = D + ((size_t)rb * kst + kc) * TILE + g * 1024 + ch * 128 + rr * 16;
+    for (int s = 0; s < c.n; ++s) {
+        const float m = c.m[s], inv = c.inv[s], c17 = c.c17[s], c34 = c.c34[s], w = c.w[s];
+        uint32_t o[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            uint32_t r[4];
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+                const int i = 4 * j + x;
+                float t = residue(__fmaf_rn(p2[i], c34, __fmaf_rn(p1[i], c17, p0[i])), m, inv);
+                if (w != 0.0f) t = residue(t * w, m, inv);
+                r[x] = __float_as_uint(__fadd_rn(t, kRoundF));
+            }
+            o[j] = __byte_perm(__byte_perm(r[0], r[1], 0x0040), __byte_perm(r[2], r[3], 0x0040), 0x5410);
+        }
+        *reinterpret_cast<uint4*>(dst + (size_t)s * plane) = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+}
+
+// C from the K ranges' residues t_i in [0, m_i): sum t_i (M / m_i) less the multiple of M that the
+// fractions' sum names (|C| / M < 0.42, so its rounding is safe).  M / m_i in three limbs of 39 bits,
+// whose sums stay below 2^53: exact in FP64 (0.52 ms for 8192 x 2501; in 128-bit
+// integers, with the K ranges in a loop, 0.87).  Four columns per thread.
+template <int Split>
+__global__ void __launch_bounds__(256) crt_kernel(int m, int n, Crt c, int bits, const uint8_t* __restrict__ T, long long ldp,
+                           size_t plane, const double* __restrict__ SA, const double* __restrict__ SB,
+                           const int* __restrict__ err, double* __restrict__ C, long long ldc)
+{
+    const int i = blockIdx.y, j0 = 4 * (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    if (j0 >= n) return;
+    const uint8_t* row = T + (size_t)i * ldp + j0;
+    double s0[4] = {0.0, 0.0, 0.0, 0.0}, s1[4] = {0.0, 0.0, 0.0, 0.0}, s2[4] = {0.0, 0.0, 0.0, 0.0};
+    float f[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll 5
+    for (int q = 0; q < c.n; ++q) {
+        unsigned t[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+        for (int s = 0; s < Split; ++s) {
+            const uint32_t b = *reinterpret_cast<const uint32_t*>(row + ((size_t)s * c.n + q) * plane);
+#pragma unroll
+            for (int x = 0; x < 4; ++x) t[x] += (b >> (8 * x)) & 0xffu;
+        }
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {  // (t < 2^10)
+            const double d = __hiloint2double(0x43300000, (int)t[x]) - 4503599627370496.0;
+            s0[x] += c.P[q][0] * d;
+            s1[x] += c.P[q][1] * d;
+            s2[x] += c.P[q][2] * d;
+            f[x] = __fmaf_rn(__uint_as_float(0x4b000000u | t[x]) - 8388608.0f, c.inv[q], f[x]);
+        }
+    }
+    const double unit = ldexp(1.0, -2 * bits);  // the product of the operands' last digits
+    const bool bad = *err != 0;
+    constexpr long long kMask = (1ll << 39) - 1;
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+        if (j0 + x >= n) break;
+        const double r = rint((double)f[x]);
+        long long a0 = (long long)(s0[x] - r * c.M[0]), a1 = (long long)(s1[x] - r * c.M[1]),
+                  a2 = (long long)(s2[x] - r * c.M[2]);
+        auto carry = [&]() {
+            a1 += a0 >> 39;
+            a0 &= kMask;
+            a2 += a1 >> 39;
+            a1 &= kMask;
+        };
+        carry();
+        const bool negative = a2 < 0;
+        if (negative) {
+            a0 = -a0;
+            a1 = -a1;
+            a2 = -a2;
+            carry();
+        }
+        const double d = fma((double)a2, 0x1p78, fma((double)a1, 0x1p39, (double)a0));
+        const double v = (((negative ? -d : d) * unit) * SB[j0 + x]) * SA[i];
+        C[(size_t)i * ldc + j0 + x] = bad ? __longlong_as_double(0x7ff8000000000000ll) : v;
+    }
+}
+
 // ---- the tensor-core product ----------------------------------------------------------------
 
+// Residues: level lev is plane lev of A times plane lev of B, and what is stored of its sums is their
+// residue modulo the chunk's modulus lev, a byte (modulus `first + lev` of `total` in T)
+template <bool Residues>
 __global__ void __launch_bounds__(THREADS, 1)
     gemm_kernel(int mt_count, int nt_count, int kst, int split, int slices, size_t a_plane, size_t b_plane,
                 const uint8_t* __restrict__ DA, const uint8_t* __restrict__ DB, int* __restrict__ levels,
-                long long ldp, int* __restrict__ err)
+                long long ldp, int* __restrict__ err, Chunk chunk, int first_mod, int total,
+                uint8_t* __restrict__ T)
 {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -364,9 +577,9 @@ __global__ void __launch_bounds__(THREADS, 1)
         long long it = 0;
         bool ok = true;
         for (int lev = 0; lev < slices && ok; ++lev)
-            for (int s = 0; s <= lev && ok; ++s) {
+            for (int s = Residues ? lev : 0; s <= lev && ok; ++s) {
                 const uint8_t* pa = DA + (size_t)s * a_plane + (size_t)mt * kst * TILE;
-                const uint8_t* pb = DB + (size_t)(lev - s) * b_plane + (size_t)nt * kst * TILE;
+                const uint8_t* pb = DB + (size_t)(Residues ? lev : lev - s) * b_plane + (size_t)nt * kst * TILE;
                 for (int st = st0; st < st1; ++st, ++it) {
                     const int slot = (int)(it % STAGES);
                     const long long use = it / STAGES;
@@ -402,7 +615,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             }
             tc_fence_after();
             bool first = true;
-            for (int s = 0; s <= lev && ok; ++s)
+            for (int s = Residues ? lev : 0; s <= lev && ok; ++s)
                 for (int st = st0; st < st1; ++st, ++it) {
                     const int slot = (int)(it % STAGES);
                     const long long use = it / STAGES;
@@ -456,6 +669,30 @@ __global__ void __launch_bounds__(THREADS, 1)
                     uint32_t r[32];
                     tmem_ld32(tbase + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(h * 256 + c0), r);
                     tmem_wait_ld(r);
+                    if constexpr (Residues) {
+                        // |sum| < 2^28.1: three single-precision roundings of a quotient below 2^20.6
+                        // move it by less than 0.3, so |v - q m| < 0.8 m
+                        const int mod = (int)chunk.m[lev];
+                        const float inv = chunk.inv[lev];
+                        uint32_t o[8];
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            uint32_t w = 0;
+#pragma unroll
+                            for (int x = 0; x < 4; ++x) {
+                                const int v = (int)r[4 * j + x];
+                                int t = v - __float2int_rn(__int2float_rn(v) * inv) * mod;
+                                t += t < 0 ? mod : 0;
+                                w |= (uint32_t)t << (8 * x);
+                            }
+                            o[j] = w;
+                        }
+                        uint4* o4 = reinterpret_cast<uint4*>(
+                            T + (((size_t)sp * total + first_mod + lev) * mt_count * BM + row) * ldp + (size_t)nt * BN + c0);
+                        o4[0] = make_uint4(o[0], o[1], o[2], o[3]);
+                        o4[1] = make_uint4(o[4], o[5], o[6], o[7]);
+                        continue;
+                    }
                     uint4* o4 = reinterpret_cast<uint4*>(orow + c0);
 #pragma unroll
                     for (int j = 0; j < 8; ++j) o4[j] = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
@@ -519,8 +756,10 @@ int32_t run(int m, int n, int k, const double* A, int64_t lda, bool trans_a, con
     {
         std::lock_guard<std::mutex> lock(g_attr_mu);
         if (!g_attr_set[dev]) {
-            if (cudaFuncSetAttribute(gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) !=
-                cudaSuccess)
+            if (cudaFuncSetAttribute(gemm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) !=
+                    cudaSuccess ||
+                cudaFuncSetAttribute(gemm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) !=
+                    cudaSuccess)
                 return DISCOEB_ECUDA;
             g_attr_set[dev] = true;
         }
@@ -543,12 +782,44 @@ int32_t run(int m, int n, int k, const double* A, int64_t lda, bool trans_a, con
     else
         row_scale_kernel<<<g.nt * BN, 256, 0, s>>>(n, k, B, ldb, eb, sb);
     const long long ua = (long long)g.mt * BM * g.kst * (BKB / 16), ub = (long long)g.nt * BN * g.kst * (BKB / 16);
+    const Crt crt = residue_form(g);
+    if (crt.n > 0) {
+        uint8_t* T = reinterpret_cast<uint8_t*>(levels);  // (a byte per modulus where the digits keep 4 per level)
+        auto even = [](const double* X, int64_t ld, bool trans) {
+            return !trans && (ld & 1) == 0 && (reinterpret_cast<uintptr_t>(X) & 15u) == 0;
+        };
+        const int bits = 7 * (slices - 1), chunks = (crt.n + slices - 1) / slices;
+        for (int x = 0, first = 0; x < chunks; ++x) {
+            Chunk c{};
+            c.n = (crt.n - first + chunks - x - 1) / (chunks - x);
+            for (int i = 0; i < c.n; ++i) set_modulus(c, i, crt.m[first + i]);
+            residue_kernel<<<(unsigned)((ua + 255) / 256), 256, 0, s>>>(m, k, A, lda, trans_a, even(A, lda, trans_a), ea, sa,
+                                                                        g.kst, ua, bits + 7, c, g.a_plane, da);
+            for (int i = 0; i < c.n; ++i) c.w[i] = (float)crt.w[first + i];
+            residue_kernel<<<(unsigned)((ub + 255) / 256), 256, 0, s>>>(n, k, B, ldb, trans_b, even(B, ldb, trans_b), eb, sb,
+                                                                        g.kst, ub, bits + 7, c, g.b_plane, db);
+            gemm_kernel<true><<<(unsigned)(g.mt * g.nt * g.split), THREADS, SMEM_BYTES, s>>>(
+                g.mt, g.nt, g.kst, g.split, c.n, g.a_plane, g.b_plane, da, db, nullptr, g.ldp, err, c, first, crt.n, T);
+            first += c.n;
+        }
+        const auto crt_k = g.split == 1   ? crt_kernel<1>
+                           : g.split == 2 ? crt_kernel<2>
+                           : g.split == 3 ? crt_kernel<3>
+                                          : crt_kernel<4>;
+        for (int i0 = 0; i0 < m; i0 += 65535) {  // (the grid's second dimension ends there)
+            const int rows = std::min(m - i0, 65535);
+            crt_k<<<dim3((unsigned)((n + 1023) / 1024), (unsigned)rows), 256, 0, s>>>(
+                rows, n, crt, bits, T + (size_t)i0 * g.ldp, g.ldp, (size_t)g.mt * BM * g.ldp, sa + i0, sb, err,
+                C + (size_t)i0 * ldc, ldc);
+        }
+        return cudaGetLastError() == cudaSuccess ? DISCOEB_SUCCESS : DISCOEB_ECUDA;
+    }
     slice_kernel<<<(unsigned)((ua + 255) / 256), 256, 0, s>>>(m, k, A, lda, trans_a, ea, sa, g.kst, ua, slices,
                                                               g.a_plane, da);
     slice_kernel<<<(unsigned)((ub + 255) / 256), 256, 0, s>>>(n, k, B, ldb, trans_b, eb, sb, g.kst, ub, slices,
                                                               g.b_plane, db);
-    gemm_kernel<<<(unsigned)(g.mt * g.nt * g.split), THREADS, SMEM_BYTES, s>>>(
-        g.mt, g.nt, g.kst, g.split, slices, g.a_plane, g.b_plane, da, db, levels, g.ldp, err);
+    gemm_kernel<false><<<(unsigned)(g.mt * g.nt * g.split), THREADS, SMEM_BYTES, s>>>(
+        g.mt, g.nt, g.kst, g.split, slices, g.a_plane, g.b_plane, da, db, levels, g.ldp, err, Chunk{}, 0, 0, nullptr);
     const long long mn = (long long)m * n;
     reduce_kernel<<<(unsigned)((mn + 255) / 256), 256, 0, s>>>(m, n, g.split, slices, levels, g.ldp,
                                                                (long long)g.mt * BM * g.ldp, sa, sb, err, C, ldc);
