@@ -40,16 +40,16 @@ import numpy as np  # noqa: E402
 
 METRIC = "fwd+adjoint k-mode solves/s at ≤1e-4 rel err vs FP64 oracle; ms per cosmology"
 # DRAM bytes of one launch per mode, from an ncu capture of a 48-mode case of the same kernel
-# (dram__bytes_read.sum + dram__bytes_write.sum: jvp_block_kernel 1.566 MB, fwd_structured_kernel
-# 0.304 MB), scaled by the number of modes: the initial states, their tangents and the outputs grow
+# (dram__bytes_read.sum + dram__bytes_write.sum: jvp_warps_kernel 2.73 MB, fwd_block_kernel
+# 0.298 MB), scaled by the number of modes: the initial states, their tangents and the outputs grow
 # with it, the tables are shared (so this slightly overstates a full launch)
-DRAM_BYTES_PER_MODE = {"fwd+grad": 1.566e6 / 48, "forward": 0.304e6 / 48}
+DRAM_BYTES_PER_MODE = {"fwd+grad": 2.73e6 / 48, "forward": 0.298e6 / 48}
 # FP64 work per step attempt, counted by ncu on a 48-mode launch of the same kernel (thread-level
 # smsp__sass_thread_inst_executed_op_{dadd,dmul,dfma}_pred_on.sum, a DFMA counted as two flops,
-# over the launch's step attempts): jvp_block_kernel 5.526e9 + 14.086e9 + 2 x 15.101e9 = 4.982e10
-# flops over 19187 attempts; fwd_structured_kernel 0.4558e9 + 0.9701e9 + 2 x 1.4198e9 = 4.2655e9 flops over
+# over the launch's step attempts): jvp_warps_kernel 1.926e9 + 3.851e9 + 2 x 5.970e9 = 1.7717e10
+# flops over 19187 attempts; fwd_block_kernel 0.4077e9 + 1.0711e9 + 2 x 1.3852e9 = 4.2493e9 flops over
 # 19187 attempts.  Scaled by the measured attempts of the timed launch.
-FP64_FLOPS_PER_ATTEMPT = {"fwd+grad": 4.9815e10 / 19187, "forward": 4.2655e9 / 19187}
+FP64_FLOPS_PER_ATTEMPT = {"fwd+grad": 1.7717e10 / 19187, "forward": 4.2493e9 / 19187}
 UNIT = "k-mode solves/s"
 
 

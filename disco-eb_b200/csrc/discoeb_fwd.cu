@@ -1,6 +1,9 @@
 // Forward perturbation solve on sm_100a: kernels and the C ABI (include/discoeb.h).
 //
-// Layout: one warp owns one k-mode.  Its whole working set (state, eight Rodas5 stage
+// The FP64 solves run on a block of warps per mode (solve_block.cu, tangent_block.cu) wherever that is
+// the faster form; the kernels here take the rest.
+//
+// Layout of those: one warp owns one k-mode.  Its whole working set (state, eight Rodas5 stage
 // vectors, the banded chain factors and the Woodbury blocks, 27 n doubles) lives in
 // shared memory; the four background tables are read through the read-only cache.
 // All modes of all cosmologies run in one launch; each warp takes modes from a

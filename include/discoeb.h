@@ -73,7 +73,7 @@ typedef struct {
     double rtol, atol, pcoeff, icoeff, dcoeff, factormax, factormin;
     int32_t max_steps;
     int32_t method;       /* DISCOEB_METHOD_* */
-    int32_t warps_per_block;
+    int32_t warps_per_block;  /* of the one-warp-per-mode form (large batches, mixed precision); <= 0: 1 */
     /* Poll budget of every wait between cooperating warps of one mode (discoeb_jvp): a warp that
      * polls a hand-over counter this many times without progress stops the mode with
      * DISCOEB_ABORTED instead of waiting on.  <= 0: the library default, 2^24 polls of ~100 ns
