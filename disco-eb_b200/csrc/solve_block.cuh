@@ -168,17 +168,23 @@ struct Stage {
     BgTables<double> tb;
     double a, ts;
 };
+// Who may read what, and when.  Warp 0's controller writes the fields marked (c) between barrier 1 at
+// the end of one attempt and barrier 0 at the start of the next.  Of the other warps it has then met
+// only special + rows (barrier 1) since the attempt's last stage, so these read them anywhere between
+// the two; the chains read theirs before their last barrier 11, the scale warp before it arrives at
+// barrier 10 and the prep warp before its last arrival at barriers 3..9.  What the scale or prep warp
+// needs later, while it prepares the next point, it keeps in registers.
 struct Ctl {
-    double t, h, tnext;
-    int regime, go, fresh, accepted;  // fresh: the point differs from the previous attempt's
-    int nbad_cand, nbad_start, fac_ok;
+    double t, h, tnext;               // (c)
+    int regime, go, fresh, accepted;  // (c); fresh: the point differs from the previous attempt's
+    int nbad_cand, nbad_start, fac_ok;  // (c), then counted by the attempt's warps
     double g[3], gd[3];       // metric functionals of the stage (and d/da at the point)
     double sp[16];            // special rows of the stage's right-hand side
     double dlq[DISCOEB_MAX_NQ];
     double cmat[9], gz0[4];   // C = I - G Z, G and F1 applied to stage 0's chains
-    double y0_next;           // row 0 of an accepted candidate
-    double pw[2];             // the controller's powers of the two previous errors
-    double e2, e3;            // those errors (inverse) for the prep warp
+    double y0_next;           // (c) row 0 of an accepted candidate
+    double pw[2];             // the controller's powers of the two previous errors, from the prep warp
+    double e2, e3;            // (c) those errors (inverse) for the prep warp
     double au2, al2;          // W's two entries outside the tridiagonal chains: (6, 8) and (8, 6)
     double cih[8][8], hd[8];  // C_sj / h, h d_s
 };
@@ -477,8 +483,9 @@ __device__ __forceinline__ void helper_step(const WarpTeam& tm, bool warp_a, con
                                             double k, const double* sw, const DiscoebControl& C, Shared& S, int cur,
                                             const ModeMem& M, int bg_count, int& hint, Interval& iv)
 {
-    const double t = S.c.t, h = S.c.h;
-    const int regime = S.c.regime, n = D.n;
+    // all that is read of the controller's fields, before the first barrier of the attempt
+    const double t = S.c.t, h = S.c.h, tnext = S.c.tnext;
+    const int regime = S.c.regime, n = D.n, regime_next = regime_at(P, tnext, sw);
     if (warp_a) {
         const Point& pt = S.pt[cur];
         const double igh = rcp(kR5.gamma * h), ih = rcp(h);
@@ -528,7 +535,7 @@ __device__ __forceinline__ void helper_step(const WarpTeam& tm, bool warp_a, con
             bar_sync(2, 64);
         }
         const double an = u0 + S.st[7].x0;
-        prep_point(tm, true, P, D, k, an, S.c.tnext, regime_at(P, S.c.tnext, sw), S.pt[cur ^ 1], hint);
+        prep_point(tm, true, P, D, k, an, tnext, regime_next, S.pt[cur ^ 1], hint);
     } else {
         // the controller's powers of the previous errors, known before the attempt ends
         if (tm.lane < 2) {
