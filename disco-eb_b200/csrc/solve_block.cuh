@@ -1517,6 +1517,7 @@ __device__ __forceinline__ SolveResult solve_mode_block(const DiscoebCosmo& P, c
                     go = 0;
                 }
             }
+            tm.sync();  // every lane has read the previous attempt's fields
             if (tm.leader()) {
                 if (go) {
                     S.c.t = t;

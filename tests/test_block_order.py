@@ -46,3 +46,14 @@ def test_helper_warps_read_the_controllers_fields_before_their_first_barrier():
         late = branch[re.search(r"\bbar_(sync|arrive)\(", branch).start():]
         assert not set(re.findall(r"S\.c\.(\w+)", late)) & _controller_fields()
     assert "S.c." not in _body("prep_point(")
+
+
+def test_controller_writes_its_fields_after_every_lane_has_read_the_old_ones():
+    """All lanes of warp 0 read the attempt's outcome and its leader overwrites it: the lanes meet between."""
+    text = _controller()
+    write = min(m.start() for m in re.finditer(r"S\.c\.(\w+) = ", text))
+    reads = [m.start() for m in re.finditer(r"S\.c\.(\w+)(?! = )\b", text) if m.start() < write]
+    assert reads
+    assert "tm.sync();" in text[max(reads):write]
+    leader = text.rindex("if (tm.leader()) {", 0, write)
+    assert text[:leader].rstrip().endswith("tm.sync();")
