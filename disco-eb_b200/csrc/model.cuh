@@ -47,6 +47,14 @@ DHD Dims make_dims(const DiscoebCosmo& c)
     return d;
 }
 
+// every row at the same place: kernels size their memory and threads by the first cosmology's layout
+// and solve no cosmology of another one (equal n is not enough: 17 multipoles of 5 momentum bins are
+// as many rows as 5 of 15, but not as many chains)
+DHD bool same_layout(const Dims& a, const Dims& b)
+{
+    return a.n == b.n && a.nq == b.nq && a.idxgp == b.idxgp && a.idxr == b.idxr && a.iq0 == b.iq0;
+}
+
 DHD int row_stride(const Dims& D, int i) { return (i >= D.iq0 && i < D.n - 2) ? D.nq : 1; }
 
 // ---- natural cubic spline lookup (spline_interpolation.py:132-228) ----

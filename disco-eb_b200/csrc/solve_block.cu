@@ -23,7 +23,7 @@ template <int MaxThreads, int MinBlocks, bool Record>
 __global__ void __launch_bounds__(MaxThreads, MinBlocks) fwd_block_kernel(
     const DiscoebCosmo* __restrict__ cosmos, int n_cosmo, const int32_t* __restrict__ mode_cosmo, DiscoebControl ctrl,
     const double* __restrict__ kmodes, const double* __restrict__ tau_start, const double* __restrict__ y0,
-    const double* __restrict__ sw, int n_out, const double* __restrict__ tau_out, int n0, double* y_full,
+    const double* __restrict__ sw, int n_out, const double* __restrict__ tau_out, Dims D0, double* y_full,
     double* y_out20, int32_t* status, int32_t* nsteps, blk::StepRecords rec)
 {
     extern __shared__ double smem[];
@@ -37,7 +37,7 @@ __global__ void __launch_bounds__(MaxThreads, MinBlocks) fwd_block_kernel(
     auto fill_nan = [&](int from) {
         for (int j = from; j < n_out; ++j) {
             const size_t o = (size_t)mode * n_out + j;
-            if (y_full) for (int i = tm.lane; i < n0; i += 32) y_full[o * n0 + i] = qnan;
+            if (y_full) for (int i = tm.lane; i < D0.n; i += 32) y_full[o * D0.n + i] = qnan;
             if (y_out20) for (int i = tm.lane; i < 20; i += 32) y_out20[o * 20 + i] = qnan;
         }
     };
@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(MaxThreads, MinBlocks) fwd_block_kernel(
     Dims D{};
     if (!bad) {
         D = make_dims(*P);
-        bad = D.n != n0;  // every cosmology must have the sizes of the first
+        bad = !same_layout(D, D0);  // every cosmology must have the sizes of the first
     }
     if (bad) {
         if (warp == 0) fill_nan(0);
@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(MaxThreads, MinBlocks) fwd_block_kernel(
 // asked for: one warp per (mode, output); rows never reached hold NaN and stay as they are.
 __global__ void __launch_bounds__(128) project_states_kernel(
     const DiscoebCosmo* __restrict__ cosmos, int n_cosmo, const int32_t* __restrict__ mode_cosmo, long long n_points,
-    const double* __restrict__ kmodes, int n_out, const double* __restrict__ tau_out, int n0, double* y_full,
+    const double* __restrict__ kmodes, int n_out, const double* __restrict__ tau_out, Dims D0, double* y_full,
     double* y_out20)
 {
     const long long p = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -118,7 +118,8 @@ __global__ void __launch_bounds__(128) project_states_kernel(
     if (ci < 0 || ci >= n_cosmo) return;
     const DiscoebCosmo& P = cosmos[ci];
     const Dims D = make_dims(P);
-    if (D.n != n0) return;
+    if (!same_layout(D, D0)) return;
+    const int n0 = D0.n;
     double* y = y_full + (size_t)p * n0;
     if (!(y[0] == y[0])) return;
     const double k = kmodes[mode], tau = tau_out[(size_t)ci * n_out + j];
@@ -181,12 +182,12 @@ int32_t launch_fwd(const DiscoebCosmo* cosmos, int n_cosmo, const int32_t* mode_
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return DISCOEB_ECUDA;
     kernel<<<n_modes, threads, smem, stream>>>(cosmos, n_cosmo, mode_cosmo, ctrl, kmodes, tau_start, y0, sw, n_out,
-                                        tau_out, D.n, y_full, y_out20, status, nsteps,
+                                        tau_out, D, y_full, y_out20, status, nsteps,
                                         records ? *records : StepRecords{});
     if (y_full) {
         const long long points = (long long)n_modes * n_out;
         project_states_kernel<<<(unsigned)((points + 3) / 4), 128, 0, stream>>>(cosmos, n_cosmo, mode_cosmo, points,
-                                                                                kmodes, n_out, tau_out, D.n, y_full,
+                                                                                kmodes, n_out, tau_out, D, y_full,
                                                                                 y_out20);
     }
     return cudaGetLastError() == cudaSuccess ? DISCOEB_SUCCESS : DISCOEB_ECUDA;

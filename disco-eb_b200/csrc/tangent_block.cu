@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) jvp_warps_kernel(
     Dims D{};
     if (!bad) {
         D = make_dims(*P);
-        bad = D.n != D0.n || D.iq0 != D0.iq0 || D.nq != D0.nq || D.idxgp != D0.idxgp || D.idxr != D0.idxr;
+        bad = !same_layout(D, D0);
     }
     if (bad) {  // (every cosmology must have the sizes of the first)
         if (threadIdx.x == 0 && grp == 0) {
@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) jvp_warps_kernel(
 constexpr int kProjectWarps = 6;
 __global__ void __launch_bounds__(32 * kProjectWarps) project_tangents_kernel(
     const DiscoebCosmo* __restrict__ cosmos, int n_cosmo, const int32_t* __restrict__ mode_cosmo,
-    const DiscoebTangent* __restrict__ tangents, int n_dir, int n0, int n_modes, const double* __restrict__ kmodes,
+    const DiscoebTangent* __restrict__ tangents, int n_dir, Dims D0, int n_modes, const double* __restrict__ kmodes,
     const double* __restrict__ sw, int n_out, const double* __restrict__ tau_out, const double* __restrict__ tau_out_dot,
     double* y_out, double* y_out_dot)
 {
@@ -243,8 +243,8 @@ __global__ void __launch_bounds__(32 * kProjectWarps) project_tangents_kernel(
     if (ci < 0 || ci >= n_cosmo) return;
     const DiscoebCosmo& P = cosmos[ci];
     const Dims D = make_dims(P);
-    if (D.n != n0) return;
-    const int n = n0;
+    if (!same_layout(D, D0)) return;
+    const int n = D.n;
     double *y = smem, *f = y + n, *jk = f + n + warp * n;
     double* yo = y_out + ((size_t)mode * n_out + j) * n;
     for (int i = threadIdx.x; i < n; i += blockDim.x) y[i] = yo[i];
@@ -317,7 +317,7 @@ int32_t launch_jvp_block(const DiscoebCosmo* cosmos, int n_cosmo, const int32_t*
     if (Full && y_out)
         project_tangents_kernel<<<(unsigned)((long long)n_modes * n_out), 32 * kProjectWarps,
                                   (2 + kProjectWarps) * D.n * sizeof(double), stream>>>(
-            cosmos, n_cosmo, mode_cosmo, tangents, n_dir, D.n, n_modes, kmodes, sw, n_out, tau_out, tau_out_dot, y_out,
+            cosmos, n_cosmo, mode_cosmo, tangents, n_dir, D, n_modes, kmodes, sw, n_out, tau_out, tau_out_dot, y_out,
             y_out_dot);
     return cudaGetLastError() == cudaSuccess ? DISCOEB_SUCCESS : DISCOEB_ECUDA;
 }
