@@ -253,11 +253,10 @@ __global__ void __launch_bounds__(32 * (1 + kMaxDirsPerBlock)) jvp_block_kernel(
             vf[5] = m;
             __threadfence_block();
             vf[4] = 1;
-            if (grp == 0) {
-                status[mode] = R.status;
-                nsteps[mode] = R.steps;
-            }
+            if (grp == 0) nsteps[mode] = R.steps;
         }
+        tm.sync();
+        report_status(tm, R.status, m, ns, nd, vf + 2, vf + 6, poll_budget(ctrl), groups > 1, status + mode);
         return;
     }
 
@@ -437,6 +436,9 @@ int32_t launch_jvp(const DiscoebCosmo* cosmos_dev, const DiscoebCosmo* cosmo0_ho
         return DISCOEB_ECUDA;
     const long long blocks = (long long)n_modes * ((n_dir + dpb - 1) / dpb);
     if (blocks > 0x7fffffffLL) return DISCOEB_EINVAL;
+    if (blocks > n_modes && cudaMemsetAsync(status, 0, (size_t)n_modes * sizeof(int32_t),
+                                            reinterpret_cast<cudaStream_t>(stream)) != cudaSuccess)
+        return DISCOEB_ECUDA;  // (several blocks report a mode: report_status)
     kernel<<<(unsigned)blocks, 32 * (1 + dpb), smem, reinterpret_cast<cudaStream_t>(stream)>>>(
         cosmos_dev, n_cosmo, mode_cosmo, tangents_dev, n_dir, dpb, make_dims(*cosmo0_host), *ctrl, n_modes, kmodes, tau_start, y0, y0_dot,
         switch_tau, n_out, tau_out, tau_out_dot, mem, tmem, glob ? records : nullptr, y_out, y_out_dot, status,

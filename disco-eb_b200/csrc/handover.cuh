@@ -27,4 +27,23 @@ __device__ inline bool wait_at_least(const WarpTeam& tm, volatile int* flag, int
     return __shfl_sync(0xffffffffu, ok, 0) != 0;
 }
 
+// A mode's status once its forward solve has ended with `st` (the whole warp): the steps still in the
+// slots (`total` published over `slots` of them, each taken `takers` times) are waited for, because a
+// tangent that gave up on them would leave NaN behind a forward that finished.  Where several blocks
+// share a mode (status then holds 0 before the launch), the highest code of any of them stays.
+__device__ inline void report_status(const WarpTeam& tm, int st, int total, int slots, int takers,
+                                     volatile int* consumed, volatile int* abort_flag, long long max_polls, bool shared,
+                                     int32_t* status)
+{
+    bool taken = true;
+    for (int sl = 0; sl < slots; ++sl)
+        taken = taken && wait_at_least(tm, consumed + sl, takers * ((total + slots - 1 - sl) / slots), abort_flag,
+                                       max_polls);
+    if (st == DISCOEB_OK && !taken) st = DISCOEB_ABORTED;
+    if (tm.leader()) {
+        if (shared) atomicMax(status, st);
+        else *status = st;
+    }
+}
+
 }  // namespace dscb

@@ -109,13 +109,15 @@ __global__ void __launch_bounds__(kMaxThreads, 1) jvp_warps_kernel(
         const blk::StepPublisher publish{smem + L.slot, flags, L};
         const SolveResult R = blk::solve_mode_block(*P, D, ctrl, k, tau_start[mode], swm, n_out, tout, M, S, emit,
                                                     rows_out, accept, publish);
-        if (threadIdx.x == 0) {
-            __threadfence_block();
-            flags[blk::FL_DONE] = 1;
-            if (grp == 0) {
-                status[mode] = R.status;
-                nsteps[mode] = R.steps;
+        if (warp == 0) {
+            if (tm.leader()) {
+                __threadfence_block();
+                flags[blk::FL_DONE] = 1;
+                if (grp == 0) nsteps[mode] = R.steps;
             }
+            tm.sync();
+            report_status(tm, R.status, flags[blk::FL_TOTAL], 2, nd, flags + blk::FL_CONSUMED, flags + blk::FL_ABORT,
+                          budget, groups > 1, status + mode);
         }
         return;
     }
@@ -311,6 +313,8 @@ int32_t launch_jvp_block(const DiscoebCosmo* cosmos, int n_cosmo, const int32_t*
         return DISCOEB_ECUDA;
     const long long blocks = (long long)n_modes * ((n_dir + nd - 1) / nd);
     if (blocks > 0x7fffffffLL) return DISCOEB_EINVAL;
+    if (blocks > n_modes && cudaMemsetAsync(status, 0, (size_t)n_modes * sizeof(int32_t), stream) != cudaSuccess)
+        return DISCOEB_ECUDA;  // (several blocks report a mode: report_status)
     kernel<<<(unsigned)blocks, block_threads(D) + 32 * (nd + kProducers), smem, stream>>>(
         cosmos, n_cosmo, mode_cosmo, tangents, n_dir, nd, D, ctrl, n_modes, kmodes, tau_start, y0, y0_dot, sw, n_out,
         tau_out, tau_out_dot, y_out, y_out_dot, status, nsteps);
