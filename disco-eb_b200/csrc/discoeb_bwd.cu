@@ -67,7 +67,7 @@ __device__ void record_emit(const WarpTeam& tm, const DiscoebCosmo& P, const Dim
 __global__ void __launch_bounds__(128) fwd_record_kernel(
     const DiscoebCosmo* __restrict__ cosmos, int n_cosmo, const int32_t* __restrict__ mode_cosmo, DiscoebControl ctrl,
     int n_modes, const double* __restrict__ kmodes, const double* __restrict__ tau_start, const double* __restrict__ y0,
-    const double* __restrict__ sw, int n_out, const double* __restrict__ tau_out, Dims D0, int mem_doubles, int cap,
+    const double* __restrict__ sw, int n_out, const double* __restrict__ tau_out, unsigned long long layout, int mem_doubles, int cap,
     int every, long long rec_doubles, double* records, int32_t* n_acc, double* y_out20, int32_t* status, int32_t* nsteps)
 {
     extern __shared__ double smem[];
@@ -92,7 +92,8 @@ __global__ void __launch_bounds__(128) fwd_record_kernel(
             cur = ci;
         }
         const Dims D = make_dims(*P);
-        if (!bad && !same_layout(D, D0)) bad = true;  // every cosmology must have the sizes of the first
+        // every cosmology must have the sizes of the first
+        if (!bad && (mode_mem_doubles(D) != mem_doubles || layout_key(D) != layout)) bad = true;
         if (bad) {
             fill_nan(mode, 0);
             if (tm.leader()) {
@@ -196,7 +197,7 @@ __global__ void __launch_bounds__(32 * kBwdWarps, 1) bwd_split_kernel(
     const double* __restrict__ kmodes, const double* __restrict__ tau_start, const double* __restrict__ sw, int n_out,
     const double* __restrict__ tau_out, int cap, int every, long long rec_doubles, const double* __restrict__ records,
     const int32_t* __restrict__ n_acc, const int32_t* __restrict__ fwd_status, double* ws,
-    const double* __restrict__ ybar20, Dims D0, int mem_doubles, double* y0_bar, double* tau_out_bar, double* par_bar,
+    const double* __restrict__ ybar20, unsigned long long layout, int mem_doubles, double* y0_bar, double* tau_out_bar, double* par_bar,
     double* table_bar, int tstride, int table_per_mode, int32_t* status)
 {
     extern __shared__ double smem[];
@@ -219,8 +220,9 @@ __global__ void __launch_bounds__(32 * kBwdWarps, 1) bwd_split_kernel(
     }
     if (threadIdx.x < kNFlags) flags[threadIdx.x] = 0;
     __syncthreads();
-    if (st == DISCOEB_OK && !same_layout(make_dims(*P), D0)) st = DISCOEB_BAD_INDEX;
-    const int n = D0.n;
+    if (st == DISCOEB_OK && (mode_mem_doubles(make_dims(*P)) != mem_doubles || layout_key(make_dims(*P)) != layout))
+        st = DISCOEB_BAD_INDEX;
+    const int n = (mem_doubles - 4 * kMaxSlots - 32) / 23;  // state size of the launch (mode_mem_doubles)
     if (st != DISCOEB_OK) {  // no forward to take apart: report, write NaN (the whole block returns)
         for (int i = threadIdx.x; i < n; i += blockDim.x) y0_bar[(size_t)mode * n + i] = qnan;
         for (int j = threadIdx.x; j < n_out; j += blockDim.x) tau_out_bar[(size_t)mode * n_out + j] = qnan;
@@ -561,7 +563,7 @@ int32_t discoeb_fwd_record(const DiscoebCosmo* cosmos_dev, const DiscoebCosmo* c
         return DISCOEB_ECUDA;
     const int blocks = (n_modes + wpb - 1) / wpb;
     fwd_record_kernel<<<blocks, 32 * wpb, smem, reinterpret_cast<cudaStream_t>(stream)>>>(
-        cosmos_dev, n_cosmo, mode_cosmo, *ctrl, n_modes, kmodes, tau_start, y0, switch_tau, n_out, tau_out, D, mem,
+        cosmos_dev, n_cosmo, mode_cosmo, *ctrl, n_modes, kmodes, tau_start, y0, switch_tau, n_out, tau_out, layout_key(D), mem,
         step_capacity, checkpoint_every, rec, records, n_accepted, y_out20, status, nsteps);
     return cudaGetLastError() == cudaSuccess ? DISCOEB_SUCCESS : DISCOEB_ECUDA;
 }
@@ -607,7 +609,7 @@ int32_t discoeb_bwd(const DiscoebCosmo* cosmos_dev, const DiscoebCosmo* cosmo0_h
     const long long rec = record_doubles(D.n, step_capacity, checkpoint_every);
     bwd_split_kernel<<<n_modes, 32 * kBwdWarps, smem, reinterpret_cast<cudaStream_t>(stream)>>>(
         cosmos_dev, n_cosmo, mode_cosmo, n_modes, kmodes, tau_start, switch_tau, n_out, tau_out, step_capacity,
-        checkpoint_every, rec, records, n_accepted, fwd_status, static_cast<double*>(workspace), y_out20_bar, D,
+        checkpoint_every, rec, records, n_accepted, fwd_status, static_cast<double*>(workspace), y_out20_bar, layout_key(D),
         mem, y0_bar, tau_out_bar, par_bar, table_bar, table_stride, table_per_mode ? 1 : 0, status);
     return cudaGetLastError() == cudaSuccess ? DISCOEB_SUCCESS : DISCOEB_ECUDA;
 }

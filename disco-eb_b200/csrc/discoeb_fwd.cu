@@ -40,7 +40,8 @@ __global__ void __launch_bounds__(256) fwd_structured_kernel(
     const DiscoebCosmo* __restrict__ cosmos, int n_cosmo, const int32_t* __restrict__ mode_cosmo, DiscoebControl ctrl,
     int n_modes,
     const double* __restrict__ kmodes, const double* __restrict__ tau_start, const double* __restrict__ y0,
-    const double* __restrict__ sw, int n_out, const double* __restrict__ tau_out, Dims D0, int mem_doubles, int mix_doubles,
+    const double* __restrict__ sw, int n_out, const double* __restrict__ tau_out, unsigned long long layout, int mem_doubles,
+    int mix_doubles,
     double* y_full, double* y_out20, int32_t* status, int32_t* nsteps)
 {
     extern __shared__ double smem[];
@@ -51,7 +52,7 @@ __global__ void __launch_bounds__(256) fwd_structured_kernel(
     DiscoebCosmo* P = reinterpret_cast<DiscoebCosmo*>(base);
     double* wmem = base + kCosmoDoubles;
     const int total_warps = gridDim.x * wpb;
-    const int n0 = D0.n;
+    const int n0 = (mem_doubles - 4 * kMaxSlots - 32) / 23;  // state size of the launch (mode_mem_doubles)
     const double qnan = __longlong_as_double(0x7ff8000000000000LL);
     // outputs never reached are filled with NaN so that they cannot pass for data
     auto fill_nan = [&](int mode, int from) {
@@ -78,7 +79,9 @@ __global__ void __launch_bounds__(256) fwd_structured_kernel(
         }
         const Dims D = make_dims(*P);
         const int n = D.n;
-        if (!same_layout(D, D0)) {  // every cosmology must have the sizes of the first
+        if (mode_mem_doubles(D) != mem_doubles || (TM::mixed && mixed_mem_doubles(D) != mix_doubles) ||
+            layout_key(D) != layout) {
+            // every cosmology must have the sizes of the first
             fill_nan(mode, 0);
             if (tm.leader()) {
                 status[mode] = DISCOEB_BAD_INDEX;
@@ -125,7 +128,7 @@ constexpr int kMaxDirsPerBlock = 6;
 template <bool Full, bool Split>
 __global__ void __launch_bounds__(32 * (1 + kMaxDirsPerBlock)) jvp_block_kernel(
     const DiscoebCosmo* __restrict__ cosmos, int n_cosmo, const int32_t* __restrict__ mode_cosmo,
-    const DiscoebTangent* __restrict__ tangents, int n_dir, int dpb, Dims D0,
+    const DiscoebTangent* __restrict__ tangents, int n_dir, int dpb, unsigned long long layout,
     DiscoebControl ctrl, int n_modes, const double* __restrict__ kmodes, const double* __restrict__ tau_start,
     const double* __restrict__ y0, const double* __restrict__ y0_dot, const double* __restrict__ sw, int n_out,
     const double* __restrict__ tau_out, const double* __restrict__ tau_out_dot, int mem_doubles, int tan_doubles,
@@ -146,7 +149,7 @@ __global__ void __launch_bounds__(32 * (1 + kMaxDirsPerBlock)) jvp_block_kernel(
             nsteps[mode] = 0;
         }
         // outputs of width 20 (fields) or, for Full, the state size of the first cosmology
-        const int W = Full ? D0.n : 20;
+        const int W = Full ? make_dims(cosmos[0]).n : 20;
         for (int dd = 0; dd < nd; ++dd)
             for (int i = threadIdx.x; i < n_out * W; i += blockDim.x) {
                 y_out20_dot[((size_t)(d0 + dd) * n_modes + mode) * n_out * W + i] = qn;
@@ -168,7 +171,7 @@ __global__ void __launch_bounds__(32 * (1 + kMaxDirsPerBlock)) jvp_block_kernel(
     DiscoebTangent* TNs = reinterpret_cast<DiscoebTangent*>(smem + kCosmoDoubles);
     double* fmem = smem + kCosmoDoubles + dpb * kTanDoubles;
     const int rec = mem_doubles + 4;
-    const int n0 = D0.n;
+    const int n0 = (mem_doubles - 4 * kMaxSlots - 32) / 23;  // state size (mode_mem_doubles)
     constexpr int ns = Split ? 1 : 2;            // record slots
     const int gpart = Split ? 13 * n0 : 0;       // doubles of a record in global memory
     const int spart = rec - gpart;               // doubles of a record in shared memory
@@ -195,7 +198,7 @@ __global__ void __launch_bounds__(32 * (1 + kMaxDirsPerBlock)) jvp_block_kernel(
     if (warp > nd) return;  // surplus warps of the last group
     const Dims D = make_dims(*P);
     const int n = D.n;
-    if (!same_layout(D, D0)) {  // every cosmology must have the sizes of the first
+    if (mode_mem_doubles(D) != mem_doubles || layout_key(D) != layout) {  // every cosmology must have the sizes of the first
         const double qn = __longlong_as_double(0x7ff8000000000000LL);
         if (warp == 0) {
             if (tm.leader() && grp == 0) {
@@ -204,7 +207,7 @@ __global__ void __launch_bounds__(32 * (1 + kMaxDirsPerBlock)) jvp_block_kernel(
             }
         } else {
             const int dir = d0 + warp - 1;
-            const int W = Full ? D0.n : 20;
+            const int W = Full ? make_dims(cosmos[0]).n : 20;
             for (int i = tm.lane; i < n_out * W; i += 32) {
                 y_out20_dot[((size_t)dir * n_modes + mode) * n_out * W + i] = qn;
                 if (dir == 0 && y_out20) y_out20[(size_t)mode * n_out * W + i] = qn;
@@ -440,7 +443,7 @@ int32_t launch_jvp(const DiscoebCosmo* cosmos_dev, const DiscoebCosmo* cosmo0_ho
                                             reinterpret_cast<cudaStream_t>(stream)) != cudaSuccess)
         return DISCOEB_ECUDA;  // (several blocks report a mode: report_status)
     kernel<<<(unsigned)blocks, 32 * (1 + dpb), smem, reinterpret_cast<cudaStream_t>(stream)>>>(
-        cosmos_dev, n_cosmo, mode_cosmo, tangents_dev, n_dir, dpb, make_dims(*cosmo0_host), *ctrl, n_modes, kmodes, tau_start, y0, y0_dot,
+        cosmos_dev, n_cosmo, mode_cosmo, tangents_dev, n_dir, dpb, layout_key(make_dims(*cosmo0_host)), *ctrl, n_modes, kmodes, tau_start, y0, y0_dot,
         switch_tau, n_out, tau_out, tau_out_dot, mem, tmem, glob ? records : nullptr, y_out, y_out_dot, status,
         nsteps);
     return cudaGetLastError() == cudaSuccess ? DISCOEB_SUCCESS : DISCOEB_ECUDA;
@@ -498,7 +501,8 @@ int32_t discoeb_fwd(const DiscoebCosmo* cosmos_dev, const DiscoebCosmo* cosmo0_h
         return DISCOEB_ECUDA;
     int blocks = (n_modes + wpb - 1) / wpb;
     kernel<<<blocks, 32 * wpb, smem, s>>>(cosmos_dev, n_cosmo, mode_cosmo, *ctrl, n_modes, kmodes, tau_start, y0,
-                                          switch_tau, n_out, tau_out, D, mem, mix, y_full, y_out20, status, nsteps);
+                                          switch_tau, n_out, tau_out, layout_key(D), mem, mix, y_full, y_out20, status,
+                                          nsteps);
     return cudaGetLastError() == cudaSuccess ? DISCOEB_SUCCESS : DISCOEB_ECUDA;
 }
 
