@@ -64,15 +64,18 @@ __device__ void record_emit(const WarpTeam& tm, const DiscoebCosmo& P, const Dim
     tm.sync();
 }
 
+// (gate: as fwd_structured_kernel's)
 __global__ void __launch_bounds__(128) fwd_record_kernel(
     const DiscoebCosmo* __restrict__ cosmos, int n_cosmo, const int32_t* __restrict__ mode_cosmo, DiscoebControl ctrl,
     int n_modes, const double* __restrict__ kmodes, const double* __restrict__ tau_start, const double* __restrict__ y0,
     const double* __restrict__ sw, int n_out, const double* __restrict__ tau_out, unsigned long long layout, int mem_doubles, int cap,
-    int every, long long rec_doubles, double* records, int32_t* n_acc, double* y_out20, int32_t* status, int32_t* nsteps)
+    int every, long long rec_doubles, double* records, int32_t* n_acc, double* y_out20, int32_t* status, int32_t* nsteps,
+    int gate)
 {
     extern __shared__ double smem[];
     const int warp = threadIdx.x >> 5;
     const WarpTeam tm{(int)(threadIdx.x & 31)};
+    if (gate != FormChoice::kOnly && short_chain_wins(tm, n_modes, kmodes, n_out, gate)) return;
     const int wpb = blockDim.x >> 5;
     double* base = smem + (size_t)warp * (kCosmoDoublesB + mem_doubles);
     DiscoebCosmo* P = reinterpret_cast<DiscoebCosmo*>(base);
@@ -552,19 +555,25 @@ int32_t discoeb_fwd_record(const DiscoebCosmo* cosmos_dev, const DiscoebCosmo* c
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     // a block of warps per mode, as in discoeb_fwd (32 modes to k = 1: 44.6 -> 9.9 ms), bit for bit the
-    // same; many modes keep a warp each (block_wins)
-    if (blk::smem_bytes(D) <= (size_t)max_optin && blk::block_wins(D, n_modes, sms)) {
+    // same; many modes keep a warp each (forward_choice)
+    int gate = FormChoice::kOnly;
+    if (blk::smem_bytes(D) <= (size_t)max_optin) {
+        const FormChoice form = blk::forward_choice(D, n_modes, sms);
+        gate = form.gate();
         const blk::StepRecords r{records, rec, step_capacity, checkpoint_every, n_accepted};
-        return blk::launch_fwd(cosmos_dev, n_cosmo, mode_cosmo, *ctrl, n_modes, kmodes, tau_start, y0, switch_tau,
-                               n_out, tau_out, D, nullptr, y_out20, status, nsteps, &r, sms,
-                               reinterpret_cast<cudaStream_t>(stream));
+        if (form.short_chain) {
+            rc = blk::launch_fwd(cosmos_dev, n_cosmo, mode_cosmo, *ctrl, n_modes, kmodes, tau_start, y0, switch_tau,
+                                 n_out, tau_out, D, nullptr, y_out20, status, nsteps, &r, sms, gate,
+                                 reinterpret_cast<cudaStream_t>(stream));
+            if (rc || !form.many_modes) return rc;
+        }
     }
     if (cudaFuncSetAttribute(fwd_record_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return DISCOEB_ECUDA;
     const int blocks = (n_modes + wpb - 1) / wpb;
     fwd_record_kernel<<<blocks, 32 * wpb, smem, reinterpret_cast<cudaStream_t>(stream)>>>(
         cosmos_dev, n_cosmo, mode_cosmo, *ctrl, n_modes, kmodes, tau_start, y0, switch_tau, n_out, tau_out, layout_key(D), mem,
-        step_capacity, checkpoint_every, rec, records, n_accepted, y_out20, status, nsteps);
+        step_capacity, checkpoint_every, rec, records, n_accepted, y_out20, status, nsteps, gate);
     return cudaGetLastError() == cudaSuccess ? DISCOEB_SUCCESS : DISCOEB_ECUDA;
 }
 

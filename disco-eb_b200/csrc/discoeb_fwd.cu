@@ -35,18 +35,20 @@ __device__ __forceinline__ void copy_cosmo(const WarpTeam& tm, const DiscoebCosm
     tm.sync();
 }
 
-template <class TM>
+// Gated: leaves if the block form took the launch (form_choice.cuh)
+template <class TM, bool Gated>
 __global__ void __launch_bounds__(256) fwd_structured_kernel(
     const DiscoebCosmo* __restrict__ cosmos, int n_cosmo, const int32_t* __restrict__ mode_cosmo, DiscoebControl ctrl,
     int n_modes,
     const double* __restrict__ kmodes, const double* __restrict__ tau_start, const double* __restrict__ y0,
     const double* __restrict__ sw, int n_out, const double* __restrict__ tau_out, unsigned long long layout, int mem_doubles,
-    int mix_doubles,
-    double* y_full, double* y_out20, int32_t* status, int32_t* nsteps)
+    int mix_doubles, double* y_full, double* y_out20, int32_t* status, int32_t* nsteps, int gate)
 {
     extern __shared__ double smem[];
     const int warp = threadIdx.x >> 5;
     const TM tm{(int)(threadIdx.x & 31)};
+    if constexpr (Gated)
+        if (short_chain_wins(tm, n_modes, kmodes, n_out, gate)) return;
     const int wpb = blockDim.x >> 5;
     double* base = smem + (size_t)warp * (kCosmoDoubles + mem_doubles + mix_doubles);
     DiscoebCosmo* P = reinterpret_cast<DiscoebCosmo*>(base);
@@ -132,12 +134,13 @@ __global__ void __launch_bounds__(32 * (1 + kMaxDirsPerBlock)) jvp_block_kernel(
     DiscoebControl ctrl, int n_modes, const double* __restrict__ kmodes, const double* __restrict__ tau_start,
     const double* __restrict__ y0, const double* __restrict__ y0_dot, const double* __restrict__ sw, int n_out,
     const double* __restrict__ tau_out, const double* __restrict__ tau_out_dot, int mem_doubles, int tan_doubles,
-    double* rec_glob, double* y_out20, double* y_out20_dot, int32_t* status, int32_t* nsteps)
+    double* rec_glob, double* y_out20, double* y_out20_dot, int32_t* status, int32_t* nsteps, int gate)
 {
     extern __shared__ double smem[];
     const int warp = threadIdx.x >> 5;
     WarpTeamSeq tm;
     tm.lane = (int)(threadIdx.x & 31);
+    if (gate != FormChoice::kOnly && short_chain_wins(tm, n_modes, kmodes, n_out, gate)) return;
     const int groups = (n_dir + dpb - 1) / dpb;
     const int mode = blockIdx.x / groups, grp = blockIdx.x - mode * groups;
     const int d0 = grp * dpb, nd = min(dpb, n_dir - d0);
@@ -394,6 +397,33 @@ JvpPlan jvp_plan(const DiscoebCosmo& c0, int n_dir, int n_modes)
     return p;
 }
 
+// The block of warps (nd directions a block) against jvp_block_kernel (dpb).  Its chain is a third as
+// long, but where shared memory holds few directions beside it the forward runs once more per group of
+// them.  Milliseconds, block / older, k from 1e-4 to 1, six directions, 1000 modes: twice the groups still
+// win (93 to 156 rows 275 / 370, 144 rows 262 / 364, 194 rows 290 / 834); three times and more do not
+// (161 rows 475 / 384, 121 rows of 8 bins 835 / 377, 219 rows 903 / 842), where few modes do (161 rows, 80
+// modes 37.5 / 82.2; equal k, 49 modes 90 / 192, 148 modes 286 / 205).
+// - Against the split record at one direction a block (219 rows, whole states): 600 modes to k = 0.5, 40
+//   outputs 576 / 664 (to k = 1), 320 outputs 1027 / 930, 2000 outputs 4409 / 3529, but 300 modes 505 / 522 and 80
+//   modes 703 / 803: each of the six forwards stops at every output.
+// - Many whole states favour the block, which projects them afterwards: 161 rows, 320 outputs 501 / 545.
+// - One direction asked for: the older form then has several blocks per SM (72 rows, 1000 modes 164 / 124;
+//   99 rows 173 / 179, 143 rows 164 / 213).
+FormChoice jvp_choice(const Dims& D, int n_dir, int nd, int dpb, bool split, bool full, int n_out, int n_modes, int sms)
+{
+    const int groups = (n_dir + nd - 1) / nd, older = dpb > 0 ? (n_dir + dpb - 1) / dpb : 0;
+    long long limit = n_modes;  // (the block form only)
+    if (dpb == 0) return FormChoice(n_modes, limit);
+    if (split) {
+        if (groups > 1 && nd == 1 && n_out > 128) limit = 3LL * sms / 2;
+    } else if (n_dir == 1 && D.n < 99) {
+        limit = sms;
+    } else if (groups > (full && n_out > 128 ? 3 : 2) * older) {
+        limit = 2LL * sms * older / groups;
+    }
+    return FormChoice(n_modes, limit);
+}
+
 template <bool Full>
 int32_t launch_jvp(const DiscoebCosmo* cosmos_dev, const DiscoebCosmo* cosmo0_host, int32_t n_cosmo,
                    const int32_t* mode_cosmo, const DiscoebTangent* tangents_dev, int32_t n_dir,
@@ -412,24 +442,30 @@ int32_t launch_jvp(const DiscoebCosmo* cosmos_dev, const DiscoebCosmo* cosmo0_ho
         return DISCOEB_EINVAL;
     if (ctrl->method != DISCOEB_METHOD_RODAS5_STRUCTURED) return DISCOEB_EUNSUPPORTED;
     if (!(ctrl->rtol > 0.0) || !(ctrl->atol >= 0.0) || ctrl->max_steps < 1) return DISCOEB_EINVAL;
-    int dev = 0, max_optin = 0;
+    int dev = 0, max_optin = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return DISCOEB_ECUDA;
     cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    // the block form wherever one direction fits beside the forward (fewer than six per block above
-    // ~150 rows: 219 rows one, and still 214 -> 63 ms for 80 modes); larger states keep the form below
-    size_t bsmem = 0;
-    const int bnd = blk::jvp_directions(make_dims(*cosmo0_host), n_dir < kMaxDirsPerBlock ? n_dir : kMaxDirsPerBlock,
-                                        (size_t)max_optin, bsmem);
-    if (bnd > 0)
-        return blk::launch_jvp_block<Full>(cosmos_dev, n_cosmo, mode_cosmo, tangents_dev, n_dir, bnd, bsmem,
-                                           make_dims(*cosmo0_host), *ctrl, n_modes, kmodes, tau_start, y0, y0_dot,
-                                           switch_tau, n_out, tau_out, tau_out_dot, y_out, y_out_dot, status, nsteps,
-                                           reinterpret_cast<cudaStream_t>(stream));
-    const JvpPlan plan = jvp_plan(*cosmo0_host, n_dir, n_modes);
-    if (plan.dpb < 0) return DISCOEB_ECUDA;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     // the split record is used when the caller passes room for it (discoeb_jvp_records_bytes
     // recommends it where it lets more directions share a block; a caller may pass it anyway)
+    const JvpPlan plan = jvp_plan(*cosmo0_host, n_dir, n_modes);
+    if (plan.dpb < 0) return DISCOEB_ECUDA;
     const bool glob = plan.dpb_glob >= plan.dpb && plan.split_bytes > 0 && records && records_bytes >= plan.split_bytes;
+    int gate = FormChoice::kOnly;
+    size_t bsmem = 0;
+    const Dims D = make_dims(*cosmo0_host);
+    const int bnd = blk::jvp_directions(D, n_dir < kMaxDirsPerBlock ? n_dir : kMaxDirsPerBlock, (size_t)max_optin, bsmem);
+    if (bnd > 0) {
+        const FormChoice form = jvp_choice(D, n_dir, bnd, glob ? plan.dpb_glob : plan.dpb, glob, Full, n_out, n_modes, sms);
+        gate = form.gate();
+        if (form.short_chain) {
+            rc = blk::launch_jvp_block<Full>(cosmos_dev, n_cosmo, mode_cosmo, tangents_dev, n_dir, bnd, bsmem, D, *ctrl,
+                                             n_modes, kmodes, tau_start, y0, y0_dot, switch_tau, n_out, tau_out,
+                                             tau_out_dot, y_out, y_out_dot, status, nsteps, gate,
+                                             reinterpret_cast<cudaStream_t>(stream));
+            if (rc || !form.many_modes) return rc;
+        }
+    }
     if (!glob && plan.dpb == 0) return DISCOEB_EUNSUPPORTED;
     const int dpb = glob ? plan.dpb_glob : plan.dpb;
     const size_t smem = glob ? plan.smem_glob : plan.smem;
@@ -439,13 +475,15 @@ int32_t launch_jvp(const DiscoebCosmo* cosmos_dev, const DiscoebCosmo* cosmo0_ho
         return DISCOEB_ECUDA;
     const long long blocks = (long long)n_modes * ((n_dir + dpb - 1) / dpb);
     if (blocks > 0x7fffffffLL) return DISCOEB_EINVAL;
-    if (blocks > n_modes && cudaMemsetAsync(status, 0, (size_t)n_modes * sizeof(int32_t),
-                                            reinterpret_cast<cudaStream_t>(stream)) != cudaSuccess)
-        return DISCOEB_ECUDA;  // (several blocks report a mode: report_status)
+    // (several blocks report a mode: report_status; after the block form's kernel it holds kOtherForm)
+    if (blocks > n_modes && gate == FormChoice::kOnly &&
+        cudaMemsetAsync(status, 0, (size_t)n_modes * sizeof(int32_t), reinterpret_cast<cudaStream_t>(stream)) !=
+            cudaSuccess)
+        return DISCOEB_ECUDA;
     kernel<<<(unsigned)blocks, 32 * (1 + dpb), smem, reinterpret_cast<cudaStream_t>(stream)>>>(
-        cosmos_dev, n_cosmo, mode_cosmo, tangents_dev, n_dir, dpb, layout_key(make_dims(*cosmo0_host)), *ctrl, n_modes, kmodes, tau_start, y0, y0_dot,
-        switch_tau, n_out, tau_out, tau_out_dot, mem, tmem, glob ? records : nullptr, y_out, y_out_dot, status,
-        nsteps);
+        cosmos_dev, n_cosmo, mode_cosmo, tangents_dev, n_dir, dpb, layout_key(D), *ctrl, n_modes, kmodes, tau_start, y0,
+        y0_dot, switch_tau, n_out, tau_out, tau_out_dot, mem, tmem, glob ? records : nullptr, y_out, y_out_dot, status,
+        nsteps, gate);
     return cudaGetLastError() == cudaSuccess ? DISCOEB_SUCCESS : DISCOEB_ECUDA;
 }
 
@@ -485,13 +523,22 @@ int32_t discoeb_fwd(const DiscoebCosmo* cosmos_dev, const DiscoebCosmo* cosmo0_h
     cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    // FP64: a block of warps per mode, up to the number of modes where one warp per mode has more of
-    // them in flight; the same results bit for bit
-    if (!mixed && blk::smem_bytes(D) <= (size_t)max_optin && blk::block_wins(D, n_modes, sms))
-        return blk::launch_fwd(cosmos_dev, n_cosmo, mode_cosmo, *ctrl, n_modes, kmodes, tau_start, y0, switch_tau,
-                               n_out, tau_out, D, y_full, y_out20, status, nsteps, nullptr, sms, s);
+    // FP64: a block of warps per mode, up to the work where one warp per mode has more of them in flight;
+    // the same results bit for bit
+    int gate = FormChoice::kOnly;
+    if (!mixed && blk::smem_bytes(D) <= (size_t)max_optin) {
+        const FormChoice form = blk::forward_choice(D, n_modes, sms);
+        gate = form.gate();
+        if (form.short_chain) {
+            rc = blk::launch_fwd(cosmos_dev, n_cosmo, mode_cosmo, *ctrl, n_modes, kmodes, tau_start, y0, switch_tau,
+                                 n_out, tau_out, D, y_full, y_out20, status, nsteps, nullptr, sms, gate, s);
+            if (rc || !form.many_modes) return rc;
+        }
+    }
     const size_t per_warp = (size_t)(kCosmoDoubles + mem + mix) * sizeof(double);
-    const auto kernel = mixed ? fwd_structured_kernel<WarpTeamMixed> : fwd_structured_kernel<WarpTeam>;
+    const auto kernel = mixed                        ? fwd_structured_kernel<WarpTeamMixed, false>
+                        : gate != FormChoice::kOnly ? fwd_structured_kernel<WarpTeam, true>
+                                                    : fwd_structured_kernel<WarpTeam, false>;
     int wpb = ctrl->warps_per_block > 0 ? ctrl->warps_per_block : 1;  // one mode per block: the most resident warps
     if (wpb > 8) wpb = 8;
     while (wpb > 1 && per_warp * wpb > (size_t)max_optin) --wpb;
@@ -502,7 +549,7 @@ int32_t discoeb_fwd(const DiscoebCosmo* cosmos_dev, const DiscoebCosmo* cosmo0_h
     int blocks = (n_modes + wpb - 1) / wpb;
     kernel<<<blocks, 32 * wpb, smem, s>>>(cosmos_dev, n_cosmo, mode_cosmo, *ctrl, n_modes, kmodes, tau_start, y0,
                                           switch_tau, n_out, tau_out, layout_key(D), mem, mix, y_full, y_out20, status,
-                                          nsteps);
+                                          nsteps, gate);
     return cudaGetLastError() == cudaSuccess ? DISCOEB_SUCCESS : DISCOEB_ECUDA;
 }
 

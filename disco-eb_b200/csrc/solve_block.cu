@@ -24,7 +24,7 @@ __global__ void __launch_bounds__(MaxThreads, MinBlocks) fwd_block_kernel(
     const DiscoebCosmo* __restrict__ cosmos, int n_cosmo, const int32_t* __restrict__ mode_cosmo, DiscoebControl ctrl,
     const double* __restrict__ kmodes, const double* __restrict__ tau_start, const double* __restrict__ y0,
     const double* __restrict__ sw, int n_out, const double* __restrict__ tau_out, Dims D0, double* y_full,
-    double* y_out20, int32_t* status, int32_t* nsteps, blk::StepRecords rec)
+    double* y_out20, int32_t* status, int32_t* nsteps, blk::StepRecords rec, int gate)
 {
     extern __shared__ double smem[];
     DiscoebCosmo* P = reinterpret_cast<DiscoebCosmo*>(smem);
@@ -32,6 +32,10 @@ __global__ void __launch_bounds__(MaxThreads, MinBlocks) fwd_block_kernel(
     double* wmem = smem + blk::kCosmo + blk::kSharedDoubles;
     const WarpTeam tm{(int)(threadIdx.x & 31)};
     const int mode = blockIdx.x, warp = threadIdx.x >> 5;
+    if (gate != FormChoice::kOnly && !short_chain_wins(tm, gridDim.x, kmodes, n_out, gate)) {
+        if (threadIdx.x == 0) status[mode] = kOtherForm;
+        return;
+    }
     const double qnan = __longlong_as_double(0x7ff8000000000000LL);
     // outputs never reached are filled with NaN so that they cannot pass for data
     auto fill_nan = [&](int from) {
@@ -107,8 +111,8 @@ __global__ void __launch_bounds__(MaxThreads, MinBlocks) fwd_block_kernel(
 // asked for: one warp per (mode, output); rows never reached hold NaN and stay as they are.
 __global__ void __launch_bounds__(128) project_states_kernel(
     const DiscoebCosmo* __restrict__ cosmos, int n_cosmo, const int32_t* __restrict__ mode_cosmo, long long n_points,
-    const double* __restrict__ kmodes, int n_out, const double* __restrict__ tau_out, Dims D0, double* y_full,
-    double* y_out20)
+    const double* __restrict__ kmodes, int n_out, const double* __restrict__ tau_out, Dims D0, const int32_t* __restrict__ status,
+    double* y_full, double* y_out20)
 {
     const long long p = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (p >= n_points) return;
@@ -118,7 +122,7 @@ __global__ void __launch_bounds__(128) project_states_kernel(
     if (ci < 0 || ci >= n_cosmo) return;
     const DiscoebCosmo& P = cosmos[ci];
     const Dims D = make_dims(P);
-    if (!same_layout(D, D0)) return;
+    if (!same_layout(D, D0) || status[mode] == kOtherForm) return;
     const int n0 = D0.n;
     double* y = y_full + (size_t)p * n0;
     if (!(y[0] == y[0])) return;
@@ -150,22 +154,26 @@ size_t smem_bytes(const Dims& D)
     return block_threads(D) > 512 ? ~(size_t)0 : (size_t)smem_doubles(D) * sizeof(double);
 }
 
-// A mode's solve is a serial chain, so few modes want the shortest chain (this form) and many the
-// most modes in flight (the one-warp form, 8 to 16 per SM against 2 here).  With two blocks per SM
-// the lines cross at 9 modes per SM for 31 rows, 12 for 72, 13.5 for 70 and 26 for 141; the rule
-// stays below all of them.  Milliseconds, block / one-warp: 72 rows 1024 modes 34 / 59, 2048 modes
-// 70 / 62, 6144 modes 215 / 135; 141 rows 2048 modes 73 / 109, 4096 modes 147 / 143, 12288 modes
-// 441 / 410.  Above 256 threads (50-multipole hierarchies) the block form wins at every count: 1200
-// modes 94 / 134, 2400 modes 187 / 259.
-bool block_wins(const Dims& D, int n_modes, int sms)
+// Modes of equal length per SM up to which blocks (two at a time) beat a warp per mode (8 to 16 of them),
+// from the equal times: 2.8 for 25 rows, 4.2 for 72, 5.2 for 143; with more than five momentum bins, whose
+// chains are wider, 2.7 to 4.0 for 85 to 197 rows; above 256 threads, one block per SM, 3.7 to 4.0 for 144
+// to 219 rows.  Milliseconds, block / one-warp: k from 1e-4 to 5, 72 rows, 1024 modes 43 / 98; 143 rows, 2048
+// modes 79 / 111, with 15 bins 3072 modes 186 / 118; 144 rows, 1024 modes 65 / 112, 2048 modes 128 / 115, 4096
+// modes 259 / 151; equal k, 1024 modes of 72 rows 167 / 105, of 143 rows 145 / 114, of 144 rows 212 / 120.
+// Up to 3.5 modes per SM a block has the SM to itself and modes of equal length finish in whole rounds.
+FormChoice forward_choice(const Dims& D, int n_modes, int sms)
 {
-    return block_threads(D) > 256 || 8LL * n_modes <= (24LL + D.n) * sms;
+    int tenths = 23 + D.n / 5;
+    if (chain_stride(D) != kNarrow) tenths = tenths < 29 ? tenths : 29;
+    else if (block_threads(D) > 256) tenths = 37;
+    if (2LL * n_modes <= 7LL * sms) tenths -= tenths % 10;
+    return FormChoice(n_modes, (long long)tenths * sms / 10);
 }
 
 int32_t launch_fwd(const DiscoebCosmo* cosmos, int n_cosmo, const int32_t* mode_cosmo, const DiscoebControl& ctrl,
                    int n_modes, const double* kmodes, const double* tau_start, const double* y0, const double* sw,
                    int n_out, const double* tau_out, const Dims& D, double* y_full, double* y_out20, int32_t* status,
-                   int32_t* nsteps, const StepRecords* records, int sms, cudaStream_t stream)
+                   int32_t* nsteps, const StepRecords* records, int sms, int gate, cudaStream_t stream)
 {
     const size_t smem = smem_bytes(D);
     const int threads = block_threads(D);
@@ -183,11 +191,11 @@ int32_t launch_fwd(const DiscoebCosmo* cosmos, int n_cosmo, const int32_t* mode_
         return DISCOEB_ECUDA;
     kernel<<<n_modes, threads, smem, stream>>>(cosmos, n_cosmo, mode_cosmo, ctrl, kmodes, tau_start, y0, sw, n_out,
                                         tau_out, D, y_full, y_out20, status, nsteps,
-                                        records ? *records : StepRecords{});
+                                        records ? *records : StepRecords{}, gate);
     if (y_full) {
         const long long points = (long long)n_modes * n_out;
         project_states_kernel<<<(unsigned)((points + 3) / 4), 128, 0, stream>>>(cosmos, n_cosmo, mode_cosmo, points,
-                                                                                kmodes, n_out, tau_out, D, y_full,
+                                                                                kmodes, n_out, tau_out, D, status, y_full,
                                                                                 y_out20);
     }
     return cudaGetLastError() == cudaSuccess ? DISCOEB_SUCCESS : DISCOEB_ECUDA;

@@ -6,6 +6,7 @@
 #include <cstddef>
 #include <cstdint>
 
+#include "form_choice.cuh"
 #include "stepper.cuh"
 
 namespace dscb {
@@ -14,8 +15,8 @@ namespace blk {
 // dynamic shared memory of one mode's block (~0 where the state has more rows than a block takes)
 size_t smem_bytes(const Dims& D);
 
-// whether the block form solves n_modes modes on a device of that many SMs faster than a warp per mode
-bool block_wins(const Dims& D, int n_modes, int sms);
+// the block form against a warp per mode for n_modes modes on a device of that many SMs
+FormChoice forward_choice(const Dims& D, int n_modes, int sms);
 
 // where discoeb_fwd_record's steps go: per mode `doubles` from base on, cap end times, then a start
 // state every `every` steps
@@ -27,11 +28,11 @@ struct StepRecords {
 };
 
 // the FP64 solve of discoeb_fwd and, with records, of discoeb_fwd_record (arguments checked by the
-// caller); a DISCOEB_* status
+// caller); a DISCOEB_* status.  gate: FormChoice's; the caller then launches the other form after it.
 int32_t launch_fwd(const DiscoebCosmo* cosmos, int n_cosmo, const int32_t* mode_cosmo, const DiscoebControl& ctrl,
                    int n_modes, const double* kmodes, const double* tau_start, const double* y0, const double* sw,
                    int n_out, const double* tau_out, const Dims& D, double* y_full, double* y_out20, int32_t* status,
-                   int32_t* nsteps, const StepRecords* records, int sms, cudaStream_t stream);
+                   int32_t* nsteps, const StepRecords* records, int sms, int gate, cudaStream_t stream);
 
 }  // namespace blk
 }  // namespace dscb

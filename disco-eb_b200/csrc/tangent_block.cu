@@ -23,7 +23,8 @@ __global__ void __launch_bounds__(kMaxThreads, 1) jvp_warps_kernel(
     const DiscoebTangent* __restrict__ tangents, int n_dir, int nd_max, Dims D0, DiscoebControl ctrl, int n_modes,
     const double* __restrict__ kmodes, const double* __restrict__ tau_start, const double* __restrict__ y0,
     const double* __restrict__ y0_dot, const double* __restrict__ sw, int n_out, const double* __restrict__ tau_out,
-    const double* __restrict__ tau_out_dot, double* y_out, double* y_out_dot, int32_t* status, int32_t* nsteps)
+    const double* __restrict__ tau_out_dot, double* y_out, double* y_out_dot, int32_t* status, int32_t* nsteps,
+    int gate)
 {
     extern __shared__ double smem[];
     const WarpTeam tm{(int)(threadIdx.x & 31)};
@@ -31,6 +32,10 @@ __global__ void __launch_bounds__(kMaxThreads, 1) jvp_warps_kernel(
     const int groups = (n_dir + nd_max - 1) / nd_max;
     const int mode = blockIdx.x / groups, grp = blockIdx.x - mode * groups;
     const int d0 = grp * nd_max, nd = min(nd_max, n_dir - d0);
+    if (gate != FormChoice::kOnly && !short_chain_wins(tm, n_modes, kmodes, n_out, gate)) {
+        if (threadIdx.x == 0 && grp == 0) status[mode] = kOtherForm;
+        return;
+    }
     const int W = Full ? D0.n : 20;
     const double qnan = __longlong_as_double(0x7ff8000000000000LL);
     DiscoebCosmo* P = reinterpret_cast<DiscoebCosmo*>(smem);
@@ -236,7 +241,7 @@ __global__ void __launch_bounds__(32 * kProjectWarps) project_tangents_kernel(
     const DiscoebCosmo* __restrict__ cosmos, int n_cosmo, const int32_t* __restrict__ mode_cosmo,
     const DiscoebTangent* __restrict__ tangents, int n_dir, Dims D0, int n_modes, const double* __restrict__ kmodes,
     const double* __restrict__ sw, int n_out, const double* __restrict__ tau_out, const double* __restrict__ tau_out_dot,
-    double* y_out, double* y_out_dot)
+    const int32_t* __restrict__ status, double* y_out, double* y_out_dot)
 {
     extern __shared__ double smem[];
     const WarpTeam tm{(int)(threadIdx.x & 31)};
@@ -245,7 +250,7 @@ __global__ void __launch_bounds__(32 * kProjectWarps) project_tangents_kernel(
     if (ci < 0 || ci >= n_cosmo) return;
     const DiscoebCosmo& P = cosmos[ci];
     const Dims D = make_dims(P);
-    if (!same_layout(D, D0)) return;
+    if (!same_layout(D, D0) || status[mode] == kOtherForm) return;
     const int n = D.n;
     double *y = smem, *f = y + n, *jk = f + n + warp * n;
     double* yo = y_out + ((size_t)mode * n_out + j) * n;
@@ -306,7 +311,7 @@ int32_t launch_jvp_block(const DiscoebCosmo* cosmos, int n_cosmo, const int32_t*
                          const DiscoebControl& ctrl, int n_modes, const double* kmodes, const double* tau_start,
                          const double* y0, const double* y0_dot, const double* sw, int n_out, const double* tau_out,
                          const double* tau_out_dot, double* y_out, double* y_out_dot, int32_t* status, int32_t* nsteps,
-                         cudaStream_t stream)
+                         int gate, cudaStream_t stream)
 {
     const auto kernel = jvp_warps_kernel<Full>;
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
@@ -317,22 +322,22 @@ int32_t launch_jvp_block(const DiscoebCosmo* cosmos, int n_cosmo, const int32_t*
         return DISCOEB_ECUDA;  // (several blocks report a mode: report_status)
     kernel<<<(unsigned)blocks, block_threads(D) + 32 * (nd + kProducers), smem, stream>>>(
         cosmos, n_cosmo, mode_cosmo, tangents, n_dir, nd, D, ctrl, n_modes, kmodes, tau_start, y0, y0_dot, sw, n_out,
-        tau_out, tau_out_dot, y_out, y_out_dot, status, nsteps);
+        tau_out, tau_out_dot, y_out, y_out_dot, status, nsteps, gate);
     if (Full && y_out)
         project_tangents_kernel<<<(unsigned)((long long)n_modes * n_out), 32 * kProjectWarps,
                                   (2 + kProjectWarps) * D.n * sizeof(double), stream>>>(
-            cosmos, n_cosmo, mode_cosmo, tangents, n_dir, D, n_modes, kmodes, sw, n_out, tau_out, tau_out_dot, y_out,
-            y_out_dot);
+            cosmos, n_cosmo, mode_cosmo, tangents, n_dir, D, n_modes, kmodes, sw, n_out, tau_out, tau_out_dot, status,
+            y_out, y_out_dot);
     return cudaGetLastError() == cudaSuccess ? DISCOEB_SUCCESS : DISCOEB_ECUDA;
 }
 template int32_t launch_jvp_block<false>(const DiscoebCosmo*, int, const int32_t*, const DiscoebTangent*, int, int,
                                          size_t, const Dims&, const DiscoebControl&, int, const double*, const double*,
                                          const double*, const double*, const double*, int, const double*, const double*,
-                                         double*, double*, int32_t*, int32_t*, cudaStream_t);
+                                         double*, double*, int32_t*, int32_t*, int, cudaStream_t);
 template int32_t launch_jvp_block<true>(const DiscoebCosmo*, int, const int32_t*, const DiscoebTangent*, int, int,
                                         size_t, const Dims&, const DiscoebControl&, int, const double*, const double*,
                                         const double*, const double*, const double*, int, const double*, const double*,
-                                        double*, double*, int32_t*, int32_t*, cudaStream_t);
+                                        double*, double*, int32_t*, int32_t*, int, cudaStream_t);
 
 }  // namespace blk
 }  // namespace dscb
