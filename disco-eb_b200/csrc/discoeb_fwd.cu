@@ -127,10 +127,14 @@ constexpr int kMaxDirsPerBlock = 6;
 // consumed), every wait bounded (wait_at_least); if a wait gives up, the whole block stops and
 // reports DISCOEB_ABORTED.  The step sequence is the forward's only, so the tangent is the
 // derivative of the discrete solution with the accepted steps held fixed.
-template <bool Full, bool Split>
+//
+// Split and shared records give the same bits (a test compares them), which hangs on the compiler fusing the
+// same multiply-adds in both: one number for the layout instead of the sizes, or the gate's test in every
+// instantiation, turns a choice over in one of them (2e-13).
+template <bool Full, bool Split, bool Gated>
 __global__ void __launch_bounds__(32 * (1 + kMaxDirsPerBlock)) jvp_block_kernel(
     const DiscoebCosmo* __restrict__ cosmos, int n_cosmo, const int32_t* __restrict__ mode_cosmo,
-    const DiscoebTangent* __restrict__ tangents, int n_dir, int dpb, unsigned long long layout,
+    const DiscoebTangent* __restrict__ tangents, int n_dir, int dpb, Dims D0,
     DiscoebControl ctrl, int n_modes, const double* __restrict__ kmodes, const double* __restrict__ tau_start,
     const double* __restrict__ y0, const double* __restrict__ y0_dot, const double* __restrict__ sw, int n_out,
     const double* __restrict__ tau_out, const double* __restrict__ tau_out_dot, int mem_doubles, int tan_doubles,
@@ -140,7 +144,8 @@ __global__ void __launch_bounds__(32 * (1 + kMaxDirsPerBlock)) jvp_block_kernel(
     const int warp = threadIdx.x >> 5;
     WarpTeamSeq tm;
     tm.lane = (int)(threadIdx.x & 31);
-    if (gate != FormChoice::kOnly && short_chain_wins(tm, n_modes, kmodes, n_out, gate)) return;
+    if constexpr (Gated)
+        if (short_chain_wins(tm, n_modes, kmodes, n_out, gate)) return;
     const int groups = (n_dir + dpb - 1) / dpb;
     const int mode = blockIdx.x / groups, grp = blockIdx.x - mode * groups;
     const int d0 = grp * dpb, nd = min(dpb, n_dir - d0);
@@ -152,7 +157,7 @@ __global__ void __launch_bounds__(32 * (1 + kMaxDirsPerBlock)) jvp_block_kernel(
             nsteps[mode] = 0;
         }
         // outputs of width 20 (fields) or, for Full, the state size of the first cosmology
-        const int W = Full ? make_dims(cosmos[0]).n : 20;
+        const int W = Full ? D0.n : 20;
         for (int dd = 0; dd < nd; ++dd)
             for (int i = threadIdx.x; i < n_out * W; i += blockDim.x) {
                 y_out20_dot[((size_t)(d0 + dd) * n_modes + mode) * n_out * W + i] = qn;
@@ -174,7 +179,7 @@ __global__ void __launch_bounds__(32 * (1 + kMaxDirsPerBlock)) jvp_block_kernel(
     DiscoebTangent* TNs = reinterpret_cast<DiscoebTangent*>(smem + kCosmoDoubles);
     double* fmem = smem + kCosmoDoubles + dpb * kTanDoubles;
     const int rec = mem_doubles + 4;
-    const int n0 = (mem_doubles - 4 * kMaxSlots - 32) / 23;  // state size (mode_mem_doubles)
+    const int n0 = D0.n;  // state size
     constexpr int ns = Split ? 1 : 2;            // record slots
     const int gpart = Split ? 13 * n0 : 0;       // doubles of a record in global memory
     const int spart = rec - gpart;               // doubles of a record in shared memory
@@ -201,7 +206,7 @@ __global__ void __launch_bounds__(32 * (1 + kMaxDirsPerBlock)) jvp_block_kernel(
     if (warp > nd) return;  // surplus warps of the last group
     const Dims D = make_dims(*P);
     const int n = D.n;
-    if (mode_mem_doubles(D) != mem_doubles || layout_key(D) != layout) {  // every cosmology must have the sizes of the first
+    if (!same_layout(D, D0)) {  // every cosmology must have the sizes of the first
         const double qn = __longlong_as_double(0x7ff8000000000000LL);
         if (warp == 0) {
             if (tm.leader() && grp == 0) {
@@ -210,7 +215,7 @@ __global__ void __launch_bounds__(32 * (1 + kMaxDirsPerBlock)) jvp_block_kernel(
             }
         } else {
             const int dir = d0 + warp - 1;
-            const int W = Full ? make_dims(cosmos[0]).n : 20;
+            const int W = Full ? D0.n : 20;
             for (int i = tm.lane; i < n_out * W; i += 32) {
                 y_out20_dot[((size_t)dir * n_modes + mode) * n_out * W + i] = qn;
                 if (dir == 0 && y_out20) y_out20[(size_t)mode * n_out * W + i] = qn;
@@ -470,7 +475,10 @@ int32_t launch_jvp(const DiscoebCosmo* cosmos_dev, const DiscoebCosmo* cosmo0_ho
     const int dpb = glob ? plan.dpb_glob : plan.dpb;
     const size_t smem = glob ? plan.smem_glob : plan.smem;
     const int mem = plan.mem, tmem = plan.tmem;
-    auto kernel = glob ? jvp_block_kernel<Full, true> : jvp_block_kernel<Full, false>;
+    const auto pick = [&](auto shared, auto split) { return glob ? split : shared; };
+    const auto kernel = gate == FormChoice::kOnly
+                            ? pick(jvp_block_kernel<Full, false, false>, jvp_block_kernel<Full, true, false>)
+                            : pick(jvp_block_kernel<Full, false, true>, jvp_block_kernel<Full, true, true>);
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return DISCOEB_ECUDA;
     const long long blocks = (long long)n_modes * ((n_dir + dpb - 1) / dpb);
@@ -481,7 +489,7 @@ int32_t launch_jvp(const DiscoebCosmo* cosmos_dev, const DiscoebCosmo* cosmo0_ho
             cudaSuccess)
         return DISCOEB_ECUDA;
     kernel<<<(unsigned)blocks, 32 * (1 + dpb), smem, reinterpret_cast<cudaStream_t>(stream)>>>(
-        cosmos_dev, n_cosmo, mode_cosmo, tangents_dev, n_dir, dpb, layout_key(D), *ctrl, n_modes, kmodes, tau_start, y0,
+        cosmos_dev, n_cosmo, mode_cosmo, tangents_dev, n_dir, dpb, D, *ctrl, n_modes, kmodes, tau_start, y0,
         y0_dot, switch_tau, n_out, tau_out, tau_out_dot, mem, tmem, glob ? records : nullptr, y_out, y_out_dot, status,
         nsteps, gate);
     return cudaGetLastError() == cudaSuccess ? DISCOEB_SUCCESS : DISCOEB_ECUDA;
