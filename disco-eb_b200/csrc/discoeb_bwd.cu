@@ -89,14 +89,13 @@ __global__ void __launch_bounds__(128) fwd_record_kernel(
     int cur = -1;
     for (int mode = blockIdx.x * wpb + warp; mode < n_modes; mode += gridDim.x * wpb) {
         const int ci = mode_cosmo ? mode_cosmo[mode] : 0;
-        bool bad = ci < 0 || ci >= n_cosmo;
+        bool bad = bad_cosmology(cosmos, n_cosmo, ci, layout);  // (every cosmology must have the sizes of the first)
         if (!bad && ci != cur) {
             copy_cosmo_warp(tm, cosmos + ci, P);
             cur = ci;
         }
         const Dims D = make_dims(*P);
-        // every cosmology must have the sizes of the first
-        if (!bad && (mode_mem_doubles(D) != mem_doubles || layout_key(D) != layout)) bad = true;
+        if (!bad && mode_mem_doubles(D) != mem_doubles) bad = true;
         if (bad) {
             fill_nan(mode, 0);
             if (tm.leader()) {
@@ -215,7 +214,7 @@ __global__ void __launch_bounds__(32 * kBwdWarps, 1) bwd_split_kernel(
     const double qnan = __longlong_as_double(0x7ff8000000000000LL);
     const int ci = mode_cosmo ? mode_cosmo[mode] : 0;
     int st = fwd_status[mode];
-    if (ci < 0 || ci >= n_cosmo) st = DISCOEB_BAD_INDEX;
+    if (bad_cosmology(cosmos, n_cosmo, ci, layout)) st = DISCOEB_BAD_INDEX;
     if (st == DISCOEB_OK) {
         const int* src = reinterpret_cast<const int*>(cosmos + ci);
         int* dst = reinterpret_cast<int*>(P);
@@ -223,8 +222,7 @@ __global__ void __launch_bounds__(32 * kBwdWarps, 1) bwd_split_kernel(
     }
     if (threadIdx.x < kNFlags) flags[threadIdx.x] = 0;
     __syncthreads();
-    if (st == DISCOEB_OK && (mode_mem_doubles(make_dims(*P)) != mem_doubles || layout_key(make_dims(*P)) != layout))
-        st = DISCOEB_BAD_INDEX;
+    if (st == DISCOEB_OK && mode_mem_doubles(make_dims(*P)) != mem_doubles) st = DISCOEB_BAD_INDEX;
     const int n = (mem_doubles - 4 * kMaxSlots - 32) / 23;  // state size of the launch (mode_mem_doubles)
     if (st != DISCOEB_OK) {  // no forward to take apart: report, write NaN (the whole block returns)
         for (int i = threadIdx.x; i < n; i += blockDim.x) y0_bar[(size_t)mode * n + i] = qnan;

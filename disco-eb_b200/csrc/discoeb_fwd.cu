@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(256) fwd_structured_kernel(
     int cur_cosmo = -1;
     for (int mode = blockIdx.x * wpb + warp; mode < n_modes; mode += total_warps) {
         const int ci = mode_cosmo ? mode_cosmo[mode] : 0;
-        if (ci < 0 || ci >= n_cosmo) {  // invalid cosmology index: report, solve nothing
+        if (bad_cosmology(cosmos, n_cosmo, ci, layout)) {  // invalid index or other sizes: report, solve nothing
             fill_nan(mode, 0);
             if (tm.leader()) {
                 status[mode] = DISCOEB_BAD_INDEX;
@@ -81,8 +81,7 @@ __global__ void __launch_bounds__(256) fwd_structured_kernel(
         }
         const Dims D = make_dims(*P);
         const int n = D.n;
-        if (mode_mem_doubles(D) != mem_doubles || (TM::mixed && mixed_mem_doubles(D) != mix_doubles) ||
-            layout_key(D) != layout) {
+        if (mode_mem_doubles(D) != mem_doubles || (TM::mixed && mixed_mem_doubles(D) != mix_doubles)) {
             // every cosmology must have the sizes of the first
             fill_nan(mode, 0);
             if (tm.leader()) {

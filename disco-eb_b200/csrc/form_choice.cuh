@@ -42,7 +42,7 @@ struct Attempts {
     int lo, hi, at[21];  // k = 2^lo .. 2^hi
 };
 #if defined(__CUDACC__)
-static __device__ __constant__
+static __device__  // (not constant memory, which serves a warp's different entries one after the other)
 #endif
 const Attempts kAttempts = {-14, 6, {70,  83,  103, 124, 145, 207, 272,  337,  357,  353, 348,
                                      347, 353, 362, 450, 709, 1000, 1290, 1784, 2520, 3570}};

@@ -54,13 +54,22 @@ DHD bool same_layout(const Dims& a, const Dims& b)
 {
     return a.n == b.n && a.nq == b.nq && a.idxgp == b.idxgp && a.idxr == b.idxr && a.iq0 == b.iq0;
 }
-// the same in one number, for states of equal size: the one-warp kernels compare this instead (told
-// each size, the compiler keeps them apart from the state's own and the forward kernel is 4 to 8% slower:
-// 4096 modes of 72 rows 118.6 -> 122.9 ms, 1024 of 25 rows 79.3 -> 85.7)
+// the same in one number, for states of equal size
 DHD unsigned long long layout_key(const Dims& D)
 {
     return (((unsigned long long)D.nq << 12 | (unsigned)D.idxgp) << 12 | (unsigned)D.idxr) << 12 | (unsigned)D.iq0;
 }
+
+#if defined(__CUDACC__)
+// whether a mode's cosmology is none of the launch's, or has another layout than the first.  Out of line,
+// and with one number to compare, for the one-warp kernels: told each size, the compiler keeps them apart
+// from the state's own, and the forward kernel is 4 to 8% slower (4096 modes of 72 rows 118.6 -> 122.9 ms,
+// 1024 of 25 rows 79.3 -> 85.7); inlined, the number alone costs it 0.5%.
+static __device__ __noinline__ bool bad_cosmology(const DiscoebCosmo* cosmos, int n_cosmo, int ci, unsigned long long layout)
+{
+    return ci < 0 || ci >= n_cosmo || layout_key(make_dims(cosmos[ci])) != layout;
+}
+#endif
 
 DHD int row_stride(const Dims& D, int i) { return (i >= D.iq0 && i < D.n - 2) ? D.nq : 1; }
 

@@ -17,7 +17,9 @@ constexpr int kMaxThreads = 512;
 // sequence is the forward's only: the tangent is the derivative of the discrete solution with its
 // accepted steps held fixed.  Every wait between the three groups is bounded (handover.cuh); if one
 // gives up, all of them leave and the mode reports DISCOEB_ABORTED.
-template <bool Full>
+//
+// Gated: leaves if the older kernel's form has the launch (asked in every instantiation, it costs 1 to 3%).
+template <bool Full, bool Gated>
 __global__ void __launch_bounds__(kMaxThreads, 1) jvp_warps_kernel(
     const DiscoebCosmo* __restrict__ cosmos, int n_cosmo, const int32_t* __restrict__ mode_cosmo,
     const DiscoebTangent* __restrict__ tangents, int n_dir, int nd_max, Dims D0, DiscoebControl ctrl, int n_modes,
@@ -32,10 +34,11 @@ __global__ void __launch_bounds__(kMaxThreads, 1) jvp_warps_kernel(
     const int groups = (n_dir + nd_max - 1) / nd_max;
     const int mode = blockIdx.x / groups, grp = blockIdx.x - mode * groups;
     const int d0 = grp * nd_max, nd = min(nd_max, n_dir - d0);
-    if (gate != FormChoice::kOnly && !short_chain_wins(tm, n_modes, kmodes, n_out, gate)) {
-        if (threadIdx.x == 0 && grp == 0) status[mode] = kOtherForm;
-        return;
-    }
+    if constexpr (Gated)
+        if (!short_chain_wins(tm, n_modes, kmodes, n_out, gate)) {
+            if (threadIdx.x == 0 && grp == 0) status[mode] = kOtherForm;
+            return;
+        }
     const int W = Full ? D0.n : 20;
     const double qnan = __longlong_as_double(0x7ff8000000000000LL);
     DiscoebCosmo* P = reinterpret_cast<DiscoebCosmo*>(smem);
@@ -313,7 +316,7 @@ int32_t launch_jvp_block(const DiscoebCosmo* cosmos, int n_cosmo, const int32_t*
                          const double* tau_out_dot, double* y_out, double* y_out_dot, int32_t* status, int32_t* nsteps,
                          int gate, cudaStream_t stream)
 {
-    const auto kernel = jvp_warps_kernel<Full>;
+    const auto kernel = gate != FormChoice::kOnly ? jvp_warps_kernel<Full, true> : jvp_warps_kernel<Full, false>;
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return DISCOEB_ECUDA;
     const long long blocks = (long long)n_modes * ((n_dir + nd - 1) / nd);
