@@ -1362,15 +1362,16 @@ __device__ __forceinline__ void chain_step(const WarpTeam& tm, const Dims& D, Sh
 
 // publish() of a solve whose steps nobody records
 struct NoPublish {
-    __device__ __forceinline__ void copy(int, int, double, const ModeMem&, const Bands&, int, int) const {}
+    __device__ __forceinline__ void copy(int, double, const ModeMem&, const Bands&, int, int) const {}
     __device__ __forceinline__ void done(const ModeMem&) const {}
 };
 
-// The solve.  y0 is in M.y; emit(j, y, regime) runs on warp 0 with the state exactly at tout[j];
+// The solve.  y0 is in M.y; emit(j, y) runs on warp 0 with the state exactly at tout[j];
 // rows(j, i, y_i) runs on the thread that owns row i (either may do nothing); accept as in
-// solve_mode, on warp 0.  After an accepted step, publish.copy(row, position, y, M, B, thread,
-// threads) runs on every thread of special + rows while M still holds the step (all but row 0, whose
-// next stages are under way), and publish.done(M) on warp 0 when all of them are through.  Every thread of the block calls it; the result is valid on warp 0.
+// solve_mode, on warp 0.  After an accepted step, publish.copy(row, y, M, B, thread, threads) runs on
+// every thread of special + rows while M still holds the step (all but row 0, whose next stages are
+// under way), and publish.done(M) on warp 0 when all of them are through.  Every thread of the block
+// calls it; the result is valid on warp 0.
 template <class Emit, class Rows, class Accept, class Publish = NoPublish>
 __device__ __forceinline__ SolveResult solve_mode_block(const DiscoebCosmo& P, const Dims& D, const DiscoebControl& C,
                                                         double k, double t0, const double* sw, int nout,
@@ -1524,7 +1525,6 @@ __device__ __forceinline__ SolveResult solve_mode_block(const DiscoebCosmo& P, c
                     S.c.h = h;
                     S.c.tnext = tnext;
                 }
-                // the regime of the step just taken is kept for its outputs when the solve ends
                 if (go) S.c.regime = regime_at(P, t, sw);
                 S.c.go = go;
                 S.c.fresh = first || keep;
@@ -1534,7 +1534,7 @@ __device__ __forceinline__ SolveResult solve_mode_block(const DiscoebCosmo& P, c
                 S.c.fac_ok = 1;
                 S.c.e2 = prev_inv;
                 S.c.e3 = prev_prev_inv;
-                // warp 4 overwrites its stages while the rows advance
+                // the scale warp overwrites its stages while the rows advance
                 if (keep) S.c.y0_next = M.u[0] + M.K[7 * n];
             }
         }
@@ -1543,7 +1543,7 @@ __device__ __forceinline__ SolveResult solve_mode_block(const DiscoebCosmo& P, c
         const int go = S.c.go, accepted = S.c.accepted;
         if (accepted) {
             cur ^= 1;
-            publish.copy(W.i, W.pos, W.y, M, B, special ? tm.lane : 32 * (warp - 1) + tm.lane, c_rows);
+            publish.copy(W.i, W.y, M, B, special ? tm.lane : 32 * (warp - 1) + tm.lane, c_rows);
             // the state advances; each thread its own row
             if (W.i >= 0) {
                 W.y = W.i == 0 ? S.c.y0_next : W.u + M.K[7 * n + W.i];

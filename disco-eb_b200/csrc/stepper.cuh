@@ -163,11 +163,6 @@ DHD double comp(double x, int c) { return c == 0 ? x : 0.0; }
 DHD double comp(const Dual& x, int c) { return c == 0 ? x.v : (c == 1 ? x.d : 0.0); }
 DHD double comp(const HDual& x, int c) { return c == 0 ? x.v.v : (c == 1 ? x.v.d : (c == 2 ? x.d.v : x.d.d)); }
 
-// Products whose rounding a caller may pin (solve_block.cuh): by default as the source writes them.
-struct SourceRounding {
-    template <class T> static DHD T product(const T& x, const T& y) { return x * y; }
-};
-
 // ---- the 15 special rows and the metric functionals ----
 // Rows a, a h', eta, CDM, baryons, photon l <= 2, massless l <= 2 and dark energy (sp, in the
 // order of special_row) and the three functionals g = (h', eta', polter) through which the
@@ -175,7 +170,7 @@ struct SourceRounding {
 // divergence, no reductions).  Y(j) gives state entry j (type S); ivl / vl are 1/v and v of
 // momentum bin tm.lane, read through tm.bcast when tm.full().  Same equations as
 // model_synchronous (perturbations.py:88-525).
-template <class TM, class T, class S, class PR = SourceRounding, class YF>
+template <class TM, class T, class S, class YF>
 DHD void special_part(const TM& tm, const DiscoebCosmo& P, const Dims& D, const Bg<T>& b, double k, double tau,
                       YF Y, const T ivl, const T vl, T sp[15], T& g0, T& g1, T& g2)
 {
@@ -199,7 +194,7 @@ DHD void special_part(const TM& tm, const DiscoebCosmo& P, const Dims& D, const 
     const S deltag = Y(7), thetag = Y(8), y9 = Y(9);
     const S deltar = Y(idxr), thetar = Y(idxr + 1), yr2 = Y(idxr + 2);
     const S deltaq = Y(n - 2), thetaq = Y(n - 1);
-    const T rQa2 = PR::product(b.rho_Q, b.a2);
+    const T rQa2 = b.rho_Q * b.a2;
     const T dgm = b.par.grhom * (Omegac * deltac + b.par.Omegab * deltab) * b.ia;
     const T dgnu = P.grhor * P.Nmnu * drho * b.ia2;
     const T dgq = b.par.grhom * b.par.OmegaDE * deltaq * rQa2;
@@ -222,8 +217,8 @@ DHD void special_part(const TM& tm, const DiscoebCosmo& P, const Dims& D, const 
     }
     const T rptq = b.opw * b.par.grhom * b.par.OmegaDE * thetaq * rQa2;
     const T dgtheta = b.par.grhom * (Omegac * thetac + b.par.Omegab * thetab) * b.ia +
-                (4.0 / 3.0) * (P.grhog * thg + P.Neff * P.grhor * thr) * b.ia2 + P.Nmnu * P.grhor * k * fnu * b.ia2 +
-                rptq;
+                      (4.0 / 3.0) * (P.grhog * thg + P.Neff * P.grhor * thr) * b.ia2 + P.Nmnu * P.grhor * k * fnu * b.ia2 +
+                      rptq;
     const T E = (0.5 / k2) * dgtheta;
     const double cs2Q = P.cs2_DE;
     const T dgpres = (P.grhog * dge + P.grhor * P.Neff * dre) * b.ia2 * (1.0 / 3.0) + P.grhor * P.Nmnu * dp * b.ia2 +

@@ -156,7 +156,7 @@ struct StepPublisher {
     double* slots;
     volatile int* flags;
     const TanLayout& L;
-    __device__ __forceinline__ void copy(int i, int, double y, const ModeMem& M, const Bands& B, int tid, int nt) const
+    __device__ __forceinline__ void copy(int i, double y, const ModeMem& M, const Bands& B, int tid, int nt) const
     {
         double* s = slots + (flags[FL_TOTAL] & 1) * L.slot_size;
         const int n = L.n;
