@@ -196,19 +196,28 @@ struct Shared {
 constexpr int kSharedDoubles = (sizeof(Shared) + 7) / 8;
 constexpr int kCosmo = (sizeof(DiscoebCosmo) + 7) / 8;
 
-// doubles of shared memory of one mode
 // positions from one element of a chain to the next: the long chains (three and one per momentum bin),
 // rounded up to one of two widths
 constexpr int kNarrow = 8, kWide = 20;
 inline __host__ __device__ int chain_stride(const Dims& D) { return 3 + D.nq <= kNarrow ? kNarrow : kWide; }
-inline __host__ __device__ int positions_of(const Dims& D)
+// Positions per chain: the longest chain, rounded up to what the substitutions are written for.  Narrow
+// chains up to kLong take one of two lengths that keep their intermediate results in registers
+// (solve_tri_s); longer ones go by fours (solve_tri_n).  Two lengths, because a body for every four up to
+// 24 makes all states slower through their code (512 modes with tangents, 143 rows 141 -> 152 ms, 72 rows
+// 151 -> 157); rounded up to these two, chains of 4 to 8 and 13 to 16 gain over the loop (256 modes, 8
+// positions 27.8 -> 25.9 ms, 16 positions 29.8 -> 26.7; tangents of 512 modes 153 -> 148, 158 -> 156).
+constexpr int kShort = 12, kLong = 20;
+inline __host__ __device__ int chain_steps(const Dims& D)
 {
     int L = D.lmaxg;
     L = L > D.lmaxgp + 1 ? L : D.lmaxgp + 1;
     L = L > D.lmaxr + 1 ? L : D.lmaxr + 1;
     if (D.nq > 0) L = L > D.lmaxnu + 1 ? L : D.lmaxnu + 1;
-    return ((L + 3) & ~3) * chain_stride(D) + 9;
+    if (chain_stride(D) == kNarrow && L <= kLong) return L <= kShort ? kShort : kLong;
+    return (L + 3) & ~3;
 }
+inline __host__ __device__ int positions_of(const Dims& D) { return chain_steps(D) * chain_stride(D) + 9; }
+// doubles of shared memory of one mode:
 // the state vectors and stages (13 n), the functionals and scalars, the chains (8 per position)
 inline __host__ __device__ int block_mem_doubles(const Dims& D)
 {
@@ -579,11 +588,7 @@ __device__ __forceinline__ Bands make_bands(const Dims& D, double* mem)
 {
     Bands B;
     B.nl = chain_stride(D);
-    int L = D.lmaxg;
-    L = L > D.lmaxgp + 1 ? L : D.lmaxgp + 1;
-    L = L > D.lmaxr + 1 ? L : D.lmaxr + 1;
-    if (D.nq > 0) L = L > D.lmaxnu + 1 ? L : D.lmaxnu + 1;
-    B.steps = (L + 3) & ~3;
+    B.steps = chain_steps(D);
     B.pc = B.steps * B.nl + 9;
     B.row8 = (B.steps - D.lmaxg) * B.nl;
     B.E = mem;
@@ -774,8 +779,8 @@ __device__ __forceinline__ void solve_tri_s(const Bands& B, int c, double al2, d
 template <int ZS, int ES = 4> __device__ __forceinline__ void solve_tri(const Bands& B, int c, double al2, double au2, double* z)
 {
     if (B.nl != kNarrow) solve_tri_n<ZS, kWide, ES>(B, c, al2, au2, z);
-    else if (B.steps == 20) solve_tri_s<ZS, kNarrow, 20, ES>(B, c, al2, au2, z);
-    else if (B.steps == 12) solve_tri_s<ZS, kNarrow, 12, ES>(B, c, al2, au2, z);
+    else if (B.steps == kLong) solve_tri_s<ZS, kNarrow, kLong, ES>(B, c, al2, au2, z);
+    else if (B.steps == kShort) solve_tri_s<ZS, kNarrow, kShort, ES>(B, c, al2, au2, z);
     else solve_tri_n<ZS, kNarrow, ES>(B, c, al2, au2, z);
 }
 
