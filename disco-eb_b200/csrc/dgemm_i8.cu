@@ -336,6 +336,10 @@ struct Crt {
 // costs a pass over the operand's doubles per chunk and a drain of the accumulators per plane, so the
 // products must be a third fewer (6 and 7 slices) and many: milliseconds, digits / residues, at
 // 41280 (256 x 256 x 128) units 8.7 / 6.1, at 10400 2.6 / 2.2, at 2600 1.08 / 0.94, at 256 0.25 / 0.31.
+// The passes grow with the tiles of A plus those of B, the products saved with A's times B's: two more
+// passes over a tile's operand take as long as some 28 of its plane products.  7 slices (13 saved), 8192 x 301 x
+// 16386 2.49 / 2.61, 700 x 2501 x 16386 1.23 / 1.21, 4096 x 601 x 8194 1.21 / 1.09, 8192 x 1001 x 16386 4.33 / 3.98;
+// 6 slices (8 saved) 2.09 / 2.41, 1.04 / 1.12, 1.00 / 1.00, 3.57 / 3.68, and 8192 x 2501 x 4098 2.73 / 2.12.
 // v is an exact integer below 2^51 (7 slices at most), a K range at most 16512 long (gemm_kernel's
 // quotients).  The error against 64 bits is a quarter of the digits' (no dropped levels).
 Crt residue_form(const Geo& g)
@@ -347,7 +351,9 @@ Crt residue_form(const Geo& g)
     double have = 0.0;
     int n = 0;
     while (n < 16 && have < bits) have += std::log2((double)kModuli[n++]);
-    if (have < bits || range > 16512 || 3 * n > slices * (slices + 1)) return c;
+    const int pairs = slices * (slices + 1) / 2;
+    if (have < bits || range > 16512 || 3 * n > 2 * pairs) return c;
+    if (2LL * g.mt * g.nt * (pairs - n) < 57LL * (g.mt + g.nt)) return c;
     c.n = n;
     auto limbs = [](unsigned __int128 x, double (&o)[3]) {
         for (int i = 0; i < 3; ++i) o[i] = (double)(uint64_t)((x >> (39 * i)) & (((unsigned __int128)1 << 39) - 1));
