@@ -636,8 +636,9 @@ def main():
     ap.add_argument("--gemm-k", type=int, default=16386, help="--mode los-gemm: contraction length")
     ap.add_argument("--slices", type=int, default=7, help="--mode los-gemm: digit planes per operand")
     ap.add_argument("--jvp-records", default="auto", choices=["auto", "always", "never"],
-                    help="fwd+grad: where the gradient kernel keeps its step records (auto: the split record "
-                         "only where it lets more directions share a block)")
+                    help="fwd+grad: a workspace for the split step record of the kernel of large states (auto: "
+                         "where it lets more directions share a block; the block of warps, which takes the "
+                         "P(k) workloads, uses none)")
     ap.add_argument("--los-contraction", default="int8", choices=["int8", "fp64"],
                     help="--mode cmb / cmb-grad: the line of sight's frequency sum on the int8 tensor cores "
                          "(7 digit planes) or as an FP64 DGEMM")

@@ -455,8 +455,9 @@ __global__ void chi_eval_kernel(int n_rows, int n_tau, const double* __restrict_
 
 // e^{-i eta (lo + ln k)} along a row of frequencies eta = c0 q, q = thread, thread + kPhaseThreads, ...:
 // one sine and cosine per thread and row, then a rotation per frequency (a sine, a cosine, an
-// exponential and a logarithm per element bound the kernel: 8192 rows of 8193, 0.69 -> 0.39 ms; the
-// rotations' rounding stays below that of the phase itself, |phase| 2^-53)
+// exponential and a logarithm per element bound the kernel: 8192 rows of 8193, 0.69 -> 0.39 ms).  The
+// error of the angle is max(|phase|, number of rotations) 2^-53: rotations add one each, which matters
+// only where the phase itself is small, and there it is n_fft / 512 2^-53
 constexpr int kPhaseThreads = 256;
 struct PhaseWalk {
     double lk, mag, sn, cs, rs, rc;
@@ -983,10 +984,8 @@ cublasHandle_t blas_handle(int dev)
 
 inline unsigned blocks_for(long long n, int threads) { return (unsigned)((n + threads - 1) / threads); }
 
-// grid of the row kernels: columns over x (coalesced), rows over y (each block strides over rows
-// when there are more than 65535)
-// columns in x; in y as many row groups as fill the device a few times over (each thread forms its
-// column's constants once for all its rows)
+// grid of the row kernels: columns in x (coalesced); in y as many row groups as fill the device a few
+// times over (each thread forms its column's constants once for all its rows)
 inline dim3 row_grid(int n_rows, int n_cols, int threads)
 {
     const unsigned x = blocks_for(n_cols, threads);

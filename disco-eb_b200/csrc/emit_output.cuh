@@ -33,7 +33,6 @@ __device__ inline void emit_output(const WarpTeam& tm, const DiscoebCosmo& P, co
     tm.sync();
 }
 
-// TM: WarpTeam (FP64) or WarpTeamMixed (FP32 chain factors, mix_doubles more per warp)
 // Output fields and their tangents at output time j of one (mode, direction): the tangent of
 // the state at the moving output time is y' + f tau_out', then the RSA projection and the
 // output conversion in dual numbers.  y: the forward state at tau_out[j]; pf: n doubles of

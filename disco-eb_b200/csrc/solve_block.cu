@@ -178,7 +178,7 @@ int32_t launch_fwd(const DiscoebCosmo* cosmos, int n_cosmo, const int32_t* mode_
     const size_t smem = smem_bytes(D);
     const int threads = block_threads(D);
     // One block per SM has all the registers it asks for, two share the SM but spill.  Milliseconds,
-    // one / two per SM: 300 modes 15.5 / 19.8 (72 rows) and 23.5 / 29.4 (141 rows); 512 modes up to
+    // one / two per SM: 300 modes 15.5 / 19.8 (72 rows) and 23.5 / 29.4 (143 rows); 512 modes up to
     // k = 10, 30.6 / 39.0; 600 modes 26.3 / 22.4 and 30.3 / 31.2; 1024 modes 43 / 34 and 52 / 38.
     const auto pick = [&](auto one, auto two, auto wide) {
         return threads > 256 ? wide : 2LL * n_modes <= 7LL * sms ? one : two;

@@ -57,7 +57,8 @@ __device__ __forceinline__ void bar_arrive(int id, int count)
 // Where a fused multiply-add can form in more than one place of an expression the compiler's choice
 // depends on the code around it, and these few choices differ between this kernel and the one-warp
 // kernels when both are written alike.  They are pinned here to the one-warp kernels' (each found by
-// comparing single steps, bit for bit, over random states in every regime).
+// comparing single steps, bit for bit, over random states in every regime), as nvcc 12.9 compiles those:
+// another compiler may choose otherwise there, and the tests that compare the two forms then tell.
 struct Rounding {
     // 3 (a'/a)^2, from the massive-neutrino density
     static __device__ __forceinline__ double friedmann(const DiscoebCosmo& P, double grhom, double Omegam, double OmegaDE,

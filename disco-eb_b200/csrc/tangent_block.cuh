@@ -21,7 +21,7 @@
 // 41% of the instruction-cache requests miss, a miss per 16 cycles and SM, and "no instruction" is
 // the first stall (5.6 of 12 cycles per issue).  Hence the tables instead of evaluated right-hand
 // sides, one code path for all stages' sources, loops left rolled, and directions that start each
-// step together.  512 modes to k = 10, 141 rows, six directions: 253 -> 139 ms; 48 modes 73 -> 28 ms;
+// step together.  512 modes to k = 10, 143 rows, six directions: 253 -> 139 ms; 48 modes 73 -> 28 ms;
 // 80 modes of 219 rows 214 -> 63 ms.
 #pragma once
 

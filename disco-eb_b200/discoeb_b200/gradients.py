@@ -309,8 +309,8 @@ class JacobianProblem:
                 self.d_y0d.data_ptr(), self.d_sw.data_ptr(), self.nout, self.d_tout.data_ptr(),
                 self.d_toutd.data_ptr(), self.d_out.data_ptr(), self.d_outd.data_ptr(), self.d_stat[0].data_ptr(),
                 self.d_stat[1].data_ptr())
-        # large states (l_max 50): the step records in a global workspace let all directions share a
-        # block (discoeb_jvp_records); otherwise they stay in shared memory
+        # large states (l_max 50): a global workspace for the step records of the kernel that takes many
+        # modes with many outputs, and all states above 224 rows (discoeb_jvp_records)
         size_fn = (self.lib.discoeb_jvp_split_records_bytes if records == "always" else
                    self.lib.discoeb_jvp_records_bytes)
         nb = size_fn(ctypes.byref(self.dc.host), len(self.dirs), self.K)

@@ -145,8 +145,9 @@ int32_t discoeb_fwd(const DiscoebCosmo* cosmos_dev, const DiscoebCosmo* cosmo0_h
  *   tau_out_dot [n_cosmo, n_dir, n_out]  d(output times)/d(theta_d)
  *   y_out20 [n_modes, n_out, 20]     output fields (may be NULL)
  *   y_out20_dot [n_dir, n_modes, n_out, 20]  their derivatives
- * One block per mode (and group of up to 6 directions): one warp solves the forward once, the
- * others carry the tangents through its published steps; one launch. */
+ * One block per mode (and group of up to 6 directions): its first warps solve the forward once, the
+ * others carry the tangents through its published steps.  A mode of which any block gives up reports
+ * DISCOEB_ABORTED. */
 int32_t discoeb_jvp(const DiscoebCosmo* cosmos_dev, const DiscoebCosmo* cosmo0_host, int32_t n_cosmo,
                     const int32_t* mode_cosmo, const DiscoebTangent* tangents_dev, int32_t n_dir,
                     const DiscoebControl* ctrl, int32_t n_modes, const double* kmodes, const double* tau_start,
@@ -169,12 +170,15 @@ int32_t discoeb_jvp_full(const DiscoebCosmo* cosmos_dev, const DiscoebCosmo* cos
                          int32_t* status, int32_t* nsteps, void* stream);
 
 /* discoeb_jvp (full = 0) or discoeb_jvp_full (full = 1) with a caller workspace for the step
- * records that the forward warp of a block hands to its tangent warps.  The plain entries keep
- * two whole records in shared memory, which for large states (l_max 50: n = 219) leaves room for
- * only three tangent warps per block, so the forward runs twice per mode and an SM holds three
- * tangent warps.  Here one record is kept, its state and stage vectors (13 n doubles per block) in
- * the workspace and the factorisation of W in shared memory, and all six directions share a block
- * (same results bit for bit).
+ * records that the forward warp of a block hands to its tangent warps, in the kernel that takes
+ * states of more than some 224 rows, and below that the launches which the block of warps does not
+ * (many modes or outputs, where few directions fit beside the block's forward).  That kernel keeps
+ * two whole records in shared memory, which leaves room for three tangent warps per block at 219
+ * rows (l_max 50), so the forward runs twice per mode.  With the workspace it keeps one record, its
+ * state and stage vectors (13 n doubles per block) in the workspace and the factorisation of W in
+ * shared memory, and five or six directions share a block (same results bit for bit).  It pays with
+ * many output times (219 rows, 600 modes, 2000 times 5.3 -> 3.5 s; one time 0.51 -> 0.65 s).  A launch
+ * that the block of warps takes does not touch the workspace.
  * discoeb_jvp_records_bytes: the workspace size (0: the records fit with every direction in one
  * block, nothing to gain; < 0: error).  records: >= that many bytes of device memory, 16-byte
  * aligned, or NULL / too small for the shared-memory form.  Other arguments as discoeb_jvp. */

@@ -21,7 +21,7 @@ import sys
 
 import numpy as np
 
-ref = sys.argv[1] if len(sys.argv) > 1 else "/root/reference"
+ref = sys.argv[1]
 out = os.path.join(os.path.dirname(os.path.abspath(__file__)), "reference_golden.npz")
 
 
